@@ -8,270 +8,38 @@
 // the result, as singlegemm's GEMM_K = 2048 blocking does
 // (singlegemm/src/NN_mp.h:13 and its ADD_C step, singlegemm/src/kernel.h:384-400).
 //
-// Tiling: BM x BN block tile, BK-deep k slices, TM x TN outputs per thread
-// held as float4 fragments spread over the tile (rows ty*4 + i*BM/(TM/4),
-// columns tx*4 + j*BN/(TN/4)) so that a warp's float4 shared-memory reads fall
-// on distinct banks; A is staged transposed (k-major) and B as is,
-// double-buffered in shared memory with the next slice prefetched into
-// registers while the current one is consumed.
+// One tile, in several shapes (the table kShapes says what each is for):
+//
+// * BM x BN outputs per CTA, TM x TN per thread. A thread's rows are ty + i * TY
+//   and its columns tx * 4 + j * 4 * TX + {0..3}. The multiply-adds go in pairs
+//   along n (fma.rn.f32x2: two IEEE round-to-nearest FMAs per instruction, each
+//   exactly an fmaf), the A value of a pair duplicated in registers.
+// * A stays row by row in shared memory (k contiguous), so a thread reads four k
+//   of a row with one 16-byte load, any TM fits and no transpose is needed; B is
+//   read four columns at a time. A's 16-byte chunks are swizzled over the rows:
+//   the two or four consecutive rows that a warp reads fall on distinct banks.
+// * k slices of BK come in through a ring of ST buffers filled by cp.async, one
+//   barrier per slice; the fragments of k + 1 load while k computes.
+//
+// What bounds it is the FMA pipe and the instructions around it: on B200 a loop
+// of nothing but f32x2 FMAs on registers issues 114 of the 128 FMA per clock and
+// SM, and one that also reads its fragments from shared memory 83 (one warp per
+// scheduler) to 100 (two). Measured alternatives that lost: A duplicated in shared
+// memory instead of in registers (1.2-1.4x slower: twice the shared-memory
+// reads), pairs along the diagonal (no faster), scalar FMAs (0.9x), registers
+// between global and shared memory instead of cp.async (the kernel before this
+// one). Before and now, us a call (B200): 1024^3 79 -> 58 (27 -> 37 TFLOP/s),
+// 1632 x 36548 x 1024 2693 -> 2409 (51 TFLOP/s), 35 x 8457 x 2560 141 -> 99.
 #include <cuda_runtime.h>
 
 #include <cstdlib>
+#include <mutex>
 
 #include "fg_kernels.h"
 
 namespace fg {
 
-// One BM x BN output tile at (m0, n0); As / Bs are the block's double buffers.
-template <int BM, int BN, int BK, int TM, int TN, bool VEC, bool KSPLIT>
-__device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0,
-                                          float (*As)[BK][BM], float (*Bs)[BK][BN])
-{
-    constexpr int NT = (BM / TM) * (BN / TN);
-    constexpr int A_LOADS = BM * BK / NT;  // elements per thread per slice
-    constexpr int B_LOADS = BK * BN / NT;
-    static_assert(A_LOADS % 4 == 0 && B_LOADS % 4 == 0, "vector tiling");
-    static_assert(TM % 4 == 0 && TN % 4 == 0, "float4 fragments");
-
-    const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN);
-    const int ty = tid / (BN / TN);
-    const int M = p.M, N = p.N, K = p.K;
-
-    // A: a thread loads A_LOADS consecutive k of one row; B: B_LOADS consecutive n of one k row.
-    constexpr int A_TPR = BK / A_LOADS;
-    const int a_row = tid / A_TPR;
-    const int a_k = (tid % A_TPR) * A_LOADS;
-    constexpr int B_TPR = BN / B_LOADS;
-    const int b_row = tid / B_TPR;
-    const int b_n = (tid % B_TPR) * B_LOADS;
-
-    // Fragment placement: rows ty*4 + {0..3} + i*(BM/2) for the two halves of TM,
-    // columns tx*4 + {0..3} + j*(BN/2) for the two halves of TN.
-    constexpr int HM = TM / 4, HN = TN / 4;  // float4 fragments per thread per dimension
-    float ra[A_LOADS], rb[B_LOADS];
-
-    auto load_slice = [&](int k0) {
-        const int gm = m0 + a_row;
-#pragma unroll
-        for (int v = 0; v < A_LOADS; v += 4) {
-            const int gk = k0 + a_k + v;
-            if (VEC && gm < M && gk + 3 < K) {
-                float4 t = *reinterpret_cast<const float4 *>(p.A + (size_t)gm * p.lda + gk);
-                ra[v] = t.x; ra[v + 1] = t.y; ra[v + 2] = t.z; ra[v + 3] = t.w;
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    ra[v + u] = (gm < M && gk + u < K) ? p.A[(size_t)gm * p.lda + gk + u] : 0.f;
-            }
-        }
-        const int gk = k0 + b_row;
-#pragma unroll
-        for (int v = 0; v < B_LOADS; v += 4) {
-            const int gn = n0 + b_n + v;
-            if (VEC && gk < K && gn + 3 < N) {
-                float4 t = *reinterpret_cast<const float4 *>(p.B + (size_t)gk * p.ldb + gn);
-                rb[v] = t.x; rb[v + 1] = t.y; rb[v + 2] = t.z; rb[v + 3] = t.w;
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    rb[v + u] = (gk < K && gn + u < N) ? p.B[(size_t)gk * p.ldb + gn + u] : 0.f;
-            }
-        }
-    };
-    auto store_slice = [&](int buf) {
-#pragma unroll
-        for (int v = 0; v < A_LOADS; ++v) As[buf][a_k + v][a_row] = ra[v];
-#pragma unroll
-        for (int v = 0; v < B_LOADS; v += 4)
-            *reinterpret_cast<float4 *>(&Bs[buf][b_row][b_n + v]) =
-                make_float4(rb[v], rb[v + 1], rb[v + 2], rb[v + 3]);
-    };
-
-    float acc[TM][TN];
-    float sum[KSPLIT ? TM : 1][KSPLIT ? TN : 1];
-    const int kblock = (KSPLIT && p.kblock > 0 && p.kblock < K) ? p.kblock : K;
-
-    for (int kb0 = 0; kb0 < K; kb0 += kblock) {
-        const int kb1 = min(kb0 + kblock, K);
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-
-        load_slice(kb0);
-        store_slice(0);
-        __syncthreads();
-        int buf = 0;
-        for (int k0 = kb0; k0 < kb1; k0 += BK) {
-            const bool more = k0 + BK < kb1;
-            if (more) load_slice(k0 + BK);
-            // a slice past K holds zeros for both operands; skip those k so that
-            // no extra rounding step touches the sum
-            const int kend = min(BK, kb1 - k0);
-            if (kend == BK) {
-#pragma unroll
-                for (int kk = 0; kk < BK; ++kk) {
-                    float a[TM], b[TN];
-#pragma unroll
-                    for (int i = 0; i < HM; ++i) {
-                        float4 t = *reinterpret_cast<const float4 *>(
-                            &As[buf][kk][ty * 4 + i * (BM / HM)]);
-                        a[4 * i] = t.x; a[4 * i + 1] = t.y; a[4 * i + 2] = t.z; a[4 * i + 3] = t.w;
-                    }
-#pragma unroll
-                    for (int j = 0; j < HN; ++j) {
-                        float4 t = *reinterpret_cast<const float4 *>(
-                            &Bs[buf][kk][tx * 4 + j * (BN / HN)]);
-                        b[4 * j] = t.x; b[4 * j + 1] = t.y; b[4 * j + 2] = t.z; b[4 * j + 3] = t.w;
-                    }
-#pragma unroll
-                    for (int i = 0; i < TM; ++i)
-#pragma unroll
-                        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-                }
-            } else {
-                for (int kk = 0; kk < kend; ++kk) {
-                    float a[TM], b[TN];
-#pragma unroll
-                    for (int i = 0; i < HM; ++i) {
-                        float4 t = *reinterpret_cast<const float4 *>(
-                            &As[buf][kk][ty * 4 + i * (BM / HM)]);
-                        a[4 * i] = t.x; a[4 * i + 1] = t.y; a[4 * i + 2] = t.z; a[4 * i + 3] = t.w;
-                    }
-#pragma unroll
-                    for (int j = 0; j < HN; ++j) {
-                        float4 t = *reinterpret_cast<const float4 *>(
-                            &Bs[buf][kk][tx * 4 + j * (BN / HN)]);
-                        b[4 * j] = t.x; b[4 * j + 1] = t.y; b[4 * j + 2] = t.z; b[4 * j + 3] = t.w;
-                    }
-#pragma unroll
-                    for (int i = 0; i < TM; ++i)
-#pragma unroll
-                        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-                }
-            }
-            if (more) {
-                store_slice(buf ^ 1);
-                __syncthreads();
-                buf ^= 1;
-            }
-        }
-        if constexpr (KSPLIT) {
-            __syncthreads();  // buffers are refilled by the next K block
-            if (kb0 == 0) {
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) sum[i][j] = acc[i][j];
-            } else {
-#pragma unroll
-                for (int i = 0; i < TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) sum[i][j] = sum[i][j] + acc[i][j];
-            }
-        }
-    }
-    if (K == 0) {
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-    }
-
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty * 4 + (i / 4) * (BM / HM) + (i % 4);
-        if (gm >= M) continue;
-        float *c = p.C + (size_t)gm * p.ldc;
-#pragma unroll
-        for (int j = 0; j < HN; ++j) {
-            const int gn = n0 + tx * 4 + j * (BN / HN);
-            float r[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if constexpr (KSPLIT)
-                    r[u] = K > 0 ? sum[i][4 * j + u] : 0.f;
-                else
-                    r[u] = acc[i][4 * j + u];
-            }
-            if (VEC && gn + 3 < N) {
-                *reinterpret_cast<float4 *>(c + gn) = make_float4(r[0], r[1], r[2], r[3]);
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (gn + u < N) c[gn + u] = r[u];
-            }
-        }
-    }
-}
-
-template <int BM, int BN, int BK, int TM, int TN, bool VEC, bool KSPLIT>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-    ffma_sgemm_kernel(const FfmaArgs p)
-{
-    __shared__ __align__(16) float As[2][BK][BM];
-    __shared__ __align__(16) float Bs[2][BK][BN];
-    ffma_tile<BM, BN, BK, TM, TN, VEC, KSPLIT>(p, blockIdx.y * BM, blockIdx.x * BN, As, Bs);
-}
-
-// Many independent SGEMMs: CTA b works on job j with tile0[j] <= b < tile0[j + 1].
-template <int BM, int BN, int BK, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-    ffma_group_kernel(const FfmaJob *__restrict__ jobs, int njobs)
-{
-    __shared__ __align__(16) float As[2][BK][BM];
-    __shared__ __align__(16) float Bs[2][BK][BN];
-    const int b = blockIdx.x;
-    int lo = 0, hi = njobs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].tile0 <= b)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    const FfmaJob &j = jobs[lo];
-    const int t = b - j.tile0;
-    FfmaArgs p;
-    p.M = j.M; p.N = j.N; p.K = j.K;
-    p.A = j.A; p.lda = j.lda;
-    p.B = j.B; p.ldb = j.ldb;
-    p.C = j.C; p.ldc = j.ldc;
-    p.kblock = 0;
-    const int m0 = (t / j.tiles_n) * BM, n0 = (t % j.tiles_n) * BN;
-    if (j.vec)
-        ffma_tile<BM, BN, BK, TM, TN, true, false>(p, m0, n0, As, Bs);
-    else
-        ffma_tile<BM, BN, BK, TM, TN, false, false>(p, m0, n0, As, Bs);
-}
-
-int ffma_group_tile(int big) { return big ? 128 : 64; }
-
-cudaError_t launch_ffma_group(const FfmaJob *jobs_dev, int njobs, int total_tiles, int big,
-                              cudaStream_t s)
-{
-    if (njobs < 1 || total_tiles < 1) return cudaSuccess;
-    if (big)
-        ffma_group_kernel<128, 128, 16, 8, 8><<<total_tiles, 256, 0, s>>>(jobs_dev, njobs);
-    else
-        ffma_group_kernel<64, 64, 16, 4, 8><<<total_tiles, 128, 0, s>>>(jobs_dev, njobs);
-    return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------ 8 x 8 per thread
-//
-// The shape of small SGEMMs (1024^3 has 256 tiles of 64 x 64 for 148 SMs):
-// 64 x 64 tiles of 64 threads, 8 x 8 outputs per thread in four 4 x 4
-// quadrants (rows ty*4 + {0, 32}, columns tx*4 + {0, 32}), so that a thread
-// loads 8 + 8 values from shared memory per k for 64 multiply-adds (half the
-// shared-memory traffic per FMA of 4 x 8), fragments of k + 1 loaded while k
-// computes. The multiply-adds go in pairs (fma.rn.f32x2: two IEEE
-// round-to-nearest FMAs per instruction, each exactly an fmaf), so every
-// output is still one FMA per k in increasing k. Staging: the next 16-deep k
-// slice is read from global memory into registers while the current one is
-// consumed; A is stored transposed (k-major), B row by row, each quarter-warp
-// writing 128 contiguous bytes.
+namespace {
 
 __device__ __forceinline__ unsigned long long pack2(float lo, float hi)
 {
@@ -292,212 +60,419 @@ __device__ __forceinline__ void ffma2(unsigned long long &d, unsigned long long 
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-template <bool KSPLIT>
-__global__ void __launch_bounds__(64) ffma_sgemm_8x8_kernel(const FfmaArgs p)
+// E floats (4: one 16-byte copy, 1: one of 4 bytes) global -> shared, the last
+// 4 * E - bytes of them zero
+template <int E>
+__device__ __forceinline__ void copy_async(uint32_t dst, const float *src, int bytes)
 {
-    constexpr int BM = 64, BN = 64, BK = 16;
-    __shared__ __align__(16) float As[2][BK][BM];
-    __shared__ __align__(16) float Bs[2][BK][BN];
+    if constexpr (E == 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+                     : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes)
+                     : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int BM_, int BN_, int BK_, int TM_, int TN_, int ST_>
+struct Shape {
+    static constexpr int BM = BM_, BN = BN_, BK = BK_, TM = TM_, TN = TN_, ST = ST_;
+    static constexpr int TX = BN / TN, TY = BM / TM, NT = TX * TY;
+    static constexpr int STAGE = (BM + BN) * BK;  // floats per ring buffer
+    static constexpr int SMEM = ST * STAGE * 4;
+    static_assert(BM % TM == 0 && BN % TN == 0 && TN % 4 == 0, "whole fragments");
+    static_assert(BK == 16 || BK == 32, "the swizzle's row length");
+    static_assert(TX == 8 || TX == 16, "a warp holds 4 or 2 rows of column groups");
+    static_assert(NT % BK == 0 && NT % (BN / 4) == 0, "copies: a thread's k chunk and column are its own");
+};
+
+// Where the 16-byte chunk c of row r lies in A's tile: BK = 32 rows are one
+// 128-byte line each, BK = 16 rows half a line.
+template <int BK>
+__device__ __forceinline__ int a_chunk(int r, int c)
+{
+    return BK == 16 ? (c ^ ((r >> 1) & 3)) : (c ^ (r & 7));
+}
+
+// One BM x BN output tile at (m0, n0). VA / VB: A / B has 16-byte-aligned rows and
+// pointer, and comes in 16-byte copies; else in 4-byte ones. Rows past M read
+// row M - 1 and columns past N read zeros (neither is stored).
+template <class S, bool VA, bool VB>
+__device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, float *sm)
+{
+    constexpr int BM = S::BM, BN = S::BN, BK = S::BK, TM = S::TM, TN = S::TN, ST = S::ST;
+    constexpr int TX = S::TX, TY = S::TY, NT = S::NT;
     const int tid = threadIdx.x;
-    const int tx = tid & 7, ty = tid >> 3;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int tx = tid % TX, ty = tid / TX;
     const int M = p.M, N = p.N, K = p.K;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
 
-    float4 ra[4], rb[4];
-    // A: row m0 + tid, 16 k; B: rows tid / 16 + 4 v, 4 columns at (tid % 16) * 4
-    auto load_slice = [&](int k0) {
-        const int gm = m0 + tid;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int gk = k0 + 4 * v;
-            if (gm < M && gk + 3 < K) {
-                ra[v] = *reinterpret_cast<const float4 *>(p.A + (size_t)gm * p.lda + gk);
-            } else {
-                const float *a = p.A + (size_t)gm * p.lda;
-                ra[v].x = (gm < M && gk < K) ? a[gk] : 0.f;
-                ra[v].y = (gm < M && gk + 1 < K) ? a[gk + 1] : 0.f;
-                ra[v].z = (gm < M && gk + 2 < K) ? a[gk + 2] : 0.f;
-                ra[v].w = (gm < M && gk + 3 < K) ? a[gk + 3] : 0.f;
-            }
-        }
-        const int gn = n0 + (tid & 15) * 4;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int gk = k0 + (tid >> 4) + 4 * v;
-            if (gk < K && gn + 3 < N) {
-                rb[v] = *reinterpret_cast<const float4 *>(p.B + (size_t)gk * p.ldb + gn);
-            } else {
-                const float *b = p.B + (size_t)gk * p.ldb;
-                rb[v].x = (gk < K && gn < N) ? b[gn] : 0.f;
-                rb[v].y = (gk < K && gn + 1 < N) ? b[gn + 1] : 0.f;
-                rb[v].z = (gk < K && gn + 2 < N) ? b[gn + 2] : 0.f;
-                rb[v].w = (gk < K && gn + 3 < N) ? b[gn + 3] : 0.f;
-            }
-        }
+    // copies: A_C of EA floats per row of A, A_R rows per pass of the CTA; B alike
+    // (a B row may take several passes: B_P copies per thread and row group)
+    constexpr int EA = VA ? 4 : 1, EB = VB ? 4 : 1;
+    constexpr int A_C = BK / EA, A_R = NT / A_C, A_V = (BM + A_R - 1) / A_R;
+    constexpr int B_C = BN / EB, B_P = B_C > NT ? B_C / NT : 1, B_R = B_C > NT ? 1 : NT / B_C;
+    constexpr int B_V = (BK + B_R - 1) / B_R;
+    static_assert(NT % A_C == 0 && (NT % B_C == 0 || B_C % NT == 0), "whole passes");
+    const int a_r = tid / A_C, a_c = tid % A_C;
+    const int b_r = B_C > NT ? 0 : tid / B_C, b_c = tid % B_C;
+    auto a_dst = [&](int r) {
+        return sbase + (r * BK + a_chunk<BK>(r, a_c * EA / 4) * 4 + (EA == 4 ? 0 : a_c % 4)) * 4;
     };
-    auto store_slice = [&](int buf) {
+    const uint32_t a_dst0 = a_dst(a_r);
+    int b_bytes[B_P];
+    const float *b_src[B_P];
+    uint32_t b_dst[B_P];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            As[buf][4 * v + 0][tid] = ra[v].x;
-            As[buf][4 * v + 1][tid] = ra[v].y;
-            As[buf][4 * v + 2][tid] = ra[v].z;
-            As[buf][4 * v + 3][tid] = ra[v].w;
-            *reinterpret_cast<float4 *>(&Bs[buf][(tid >> 4) + 4 * v][(tid & 15) * 4]) = rb[v];
-        }
-    };
-
-    unsigned long long acc[8][4];  // row i, column pairs {0,1}, {2,3} of each quadrant
-    unsigned long long sum[KSPLIT ? 8 : 1][KSPLIT ? 4 : 1];
-    const int kblock = (KSPLIT && p.kblock > 0 && p.kblock < K) ? p.kblock : K;
-
-    for (int kb0 = 0; kb0 < K; kb0 += kblock) {
-        const int kb1 = min(kb0 + kblock, K);
+    for (int q = 0; q < B_P; ++q) {
+        const int c = (b_c + q * NT) * EB, gn = n0 + c;
+        b_bytes[q] = min(max((N - gn) * 4, 0), 4 * EB);
+        b_src[q] = p.B + (b_bytes[q] ? gn : 0) + (long)b_r * p.ldb;
+        b_dst[q] = sbase + (BM * BK + b_r * BN + c) * 4;
+    }
+    auto load = [&](int slice, int buf) {
+        const int k0 = slice * BK;
+        const uint32_t off = buf * S::STAGE * 4;
+        if (k0 + BK <= K) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+            for (int v = 0; v < A_V; ++v) {
+                const int r = a_r + v * A_R;
+                if (BM % A_R && r >= BM) break;
+                // the swizzle repeats every 8 rows
+                const uint32_t d = A_R % 8 == 0 ? a_dst0 + v * A_R * BK * 4 : a_dst(r);
+                copy_async<EA>(d + off, p.A + (long)min(m0 + r, M - 1) * p.lda + k0 + a_c * EA, 4 * EA);
+            }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-
-        load_slice(kb0);
-        store_slice(0);
-        __syncthreads();
-        int buf = 0;
-        for (int k0 = kb0; k0 < kb1; k0 += BK) {
-            const bool more = k0 + BK < kb1;
-            if (more) load_slice(k0 + BK);
-            // a slice past K holds zeros for both operands; its k are skipped so
-            // that no extra rounding step touches the sums
-            const int kend = min(BK, kb1 - k0);
-            auto step = [&](int kk) {
-                const float4 a0 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4]);
-                const float4 a1 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4 + 32]);
-                const float4 b0 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
-                const float4 b1 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4 + 32]);
-                const unsigned long long bp[4] = {pack2(b0.x, b0.y), pack2(b0.z, b0.w),
-                                                  pack2(b1.x, b1.y), pack2(b1.z, b1.w)};
-                const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            for (int q = 0; q < B_P; ++q) {
+                const float *s = b_src[q] + (long)k0 * p.ldb;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const unsigned long long ap = pack2(a[i], a[i]);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) ffma2(acc[i][j], ap, bp[j]);
+                for (int v = 0; v < B_V; ++v) {
+                    if (BK % B_R && b_r + v * B_R >= BK) break;
+                    copy_async<EB>(b_dst[q] + off + v * B_R * BN * 4, s + (long)(v * B_R) * p.ldb,
+                                   b_bytes[q]);
                 }
-            };
-            if (kend == BK) {
-#pragma unroll
-                for (int kk = 0; kk < BK; ++kk) step(kk);
-            } else {
-                for (int kk = 0; kk < kend; ++kk) step(kk);
             }
-            if (more) {
-                store_slice(buf ^ 1);
-                __syncthreads();
-                buf ^= 1;
+        } else {  // the last slice of a K that is no multiple of BK: zeros past K
+#pragma unroll
+            for (int v = 0; v < A_V; ++v) {
+                const int r = a_r + v * A_R;
+                if (BM % A_R && r >= BM) break;
+                const int gk = k0 + a_c * EA;
+                const int n = min(max((K - gk) * 4, 0), 4 * EA);
+                copy_async<EA>(a_dst(r) + off, p.A + (long)min(m0 + r, M - 1) * p.lda + (n ? gk : 0), n);
+            }
+#pragma unroll
+            for (int q = 0; q < B_P; ++q)
+#pragma unroll
+                for (int v = 0; v < B_V; ++v) {
+                    const int r = b_r + v * B_R;
+                    if (BK % B_R && r >= BK) break;
+                    const bool in = k0 + r < K;
+                    copy_async<EB>(b_dst[q] + off + v * B_R * BN * 4,
+                                   in ? b_src[q] + (long)(k0 + v * B_R) * p.ldb : p.B,
+                                   in ? b_bytes[q] : 0);
+                }
+        }
+    };
+
+    unsigned long long acc[TM][TN / 2];
+    auto clear = [&] {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
+    };
+    // the block's sums into C: stored, or added to the blocks before it
+    const bool vec_c = p.ldc % 4 == 0 && ((uintptr_t)p.C & 15) == 0;
+    auto flush = [&](bool add) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int gm = m0 + ty + i * TY;
+            if (gm >= M) continue;
+            float *c = p.C + (size_t)gm * p.ldc;
+#pragma unroll
+            for (int j = 0; j < TN / 4; ++j) {
+                const int gn = n0 + tx * 4 + j * 4 * TX;
+                float r[4];
+                unpack2(acc[i][2 * j], r[0], r[1]);
+                unpack2(acc[i][2 * j + 1], r[2], r[3]);
+                if (vec_c && gn + 3 < N) {
+                    float4 *c4 = reinterpret_cast<float4 *>(c + gn);
+                    if (add) {
+                        const float4 o = *c4;
+                        r[0] = o.x + r[0]; r[1] = o.y + r[1]; r[2] = o.z + r[2]; r[3] = o.w + r[3];
+                    }
+                    *c4 = make_float4(r[0], r[1], r[2], r[3]);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (gn + u < N) c[gn + u] = add ? c[gn + u] + r[u] : r[u];
+                }
             }
         }
-        if constexpr (KSPLIT) {
-            __syncthreads();  // buffers are refilled by the next K block
+    };
+
+    const int slices = (K + BK - 1) / BK;
+    const int per_block = p.kblock > 0 && p.kblock < K ? p.kblock / BK : slices;
+    clear();
+    if (slices == 0) flush(false);  // an empty sum
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < slices) load(s, s);
+        copy_commit();
+    }
+    int buf = 0, in_block = 0;
+#pragma unroll 1
+    for (int s = 0; s < slices; ++s) {
+        copy_wait<ST - 2>();
+        __syncthreads();  // slice s has landed; every thread has read slice s - 1
+        if (s + ST - 1 < slices) load(s + ST - 1, buf == 0 ? ST - 1 : buf - 1);
+        copy_commit();
+        const float *As = sm + buf * S::STAGE, *Bs = As + BM * BK;
+        auto a_quad = [&](int i, int q) {
+            const int r = ty + i * TY;
+            return *reinterpret_cast<const float4 *>(&As[r * BK + a_chunk<BK>(r, q) * 4]);
+        };
+        auto b_quad = [&](int k, int j) {
+            return *reinterpret_cast<const float4 *>(&Bs[k * BN + tx * 4 + j * 4 * TX]);
+        };
+        if ((s + 1) * BK <= K) {
+            float4 a[2][TM], b[2][TN / 4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    if (kb0 == 0) {
-                        sum[i][j] = acc[i][j];
-                    } else {
-                        float s0, s1, a0, a1;
-                        unpack2(sum[i][j], s0, s1);
-                        unpack2(acc[i][j], a0, a1);
-                        sum[i][j] = pack2(s0 + a0, s1 + a1);
+            for (int i = 0; i < TM; ++i) a[0][i] = a_quad(i, 0);
+#pragma unroll
+            for (int j = 0; j < TN / 4; ++j) b[0][j] = b_quad(0, j);
+#pragma unroll
+            for (int k = 0; k < BK; ++k) {
+                if (k + 1 < BK)
+#pragma unroll
+                    for (int j = 0; j < TN / 4; ++j) b[(k + 1) & 1][j] = b_quad(k + 1, j);
+                if (k % 4 == 0 && k + 4 < BK)
+#pragma unroll
+                    for (int i = 0; i < TM; ++i) a[(k / 4 + 1) & 1][i] = a_quad(i, k / 4 + 1);
+                unsigned long long bp[TN / 2];
+#pragma unroll
+                for (int j = 0; j < TN / 4; ++j) {
+                    bp[2 * j] = pack2(b[k & 1][j].x, b[k & 1][j].y);
+                    bp[2 * j + 1] = pack2(b[k & 1][j].z, b[k & 1][j].w);
+                }
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const float4 v = a[(k / 4) & 1][i];
+                    const float x = k % 4 == 0 ? v.x : k % 4 == 1 ? v.y : k % 4 == 2 ? v.z : v.w;
+                    const unsigned long long ap = pack2(x, x);
+                    // back and forth: neighbouring FMAs share an operand
+#pragma unroll
+                    for (int t = 0; t < TN / 2; ++t) {
+                        const int j = (i & 1) ? TN / 2 - 1 - t : t;
+                        ffma2(acc[i][j], ap, bp[j]);
                     }
                 }
-        }
-    }
-
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int gm = m0 + ty * 4 + (i / 4) * 32 + (i % 4);
-        if (gm >= M) continue;
-        float *c = p.C + (size_t)gm * p.ldc;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int gn = n0 + tx * 4 + h * 32;
-            float r[4];
-            unsigned long long v0 = KSPLIT ? sum[i][2 * h] : acc[i][2 * h];
-            unsigned long long v1 = KSPLIT ? sum[i][2 * h + 1] : acc[i][2 * h + 1];
-            if (K == 0) v0 = v1 = 0ull;
-            unpack2(v0, r[0], r[1]);
-            unpack2(v1, r[2], r[3]);
-            if (gn + 3 < N) {
-                *reinterpret_cast<float4 *>(c + gn) = make_float4(r[0], r[1], r[2], r[3]);
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (gn + u < N) c[gn + u] = r[u];
             }
+        } else {
+            // the k past K hold zeros for both operands; they are skipped, so that no
+            // extra rounding step (or 0 x infinity) touches the sums
+#pragma unroll 1
+            for (int k = 0; k < K - s * BK; ++k) {
+                unsigned long long bp[TN / 2];
+#pragma unroll
+                for (int j = 0; j < TN / 4; ++j) {
+                    const float4 t = b_quad(k, j);
+                    bp[2 * j] = pack2(t.x, t.y);
+                    bp[2 * j + 1] = pack2(t.z, t.w);
+                }
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const int r = ty + i * TY;
+                    const float x = As[r * BK + a_chunk<BK>(r, k / 4) * 4 + (k & 3)];
+                    const unsigned long long ap = pack2(x, x);
+#pragma unroll
+                    for (int j = 0; j < TN / 2; ++j) ffma2(acc[i][j], ap, bp[j]);
+                }
+            }
+        }
+        buf = buf + 1 == ST ? 0 : buf + 1;
+        if (++in_block == per_block || s + 1 == slices) {
+            flush(s >= per_block);
+            clear();
+            in_block = 0;
         }
     }
 }
 
-static cudaError_t launch_8x8(const FfmaArgs &a, cudaStream_t s)
+// m_fast: neighbouring CTAs share columns of B rather than rows of A
+template <class S, bool VA, bool VB>
+__global__ void __launch_bounds__(S::NT) ffma_sgemm_kernel(const FfmaArgs p, int tiles_m, int tiles_n,
+                                                           int m_fast)
 {
-    dim3 grid((a.N + 63) / 64, (a.M + 63) / 64);
-    if (a.kblock > 0 && a.kblock < a.K)
-        ffma_sgemm_8x8_kernel<true><<<grid, 64, 0, s>>>(a);
+    extern __shared__ __align__(128) float sm[];
+    const int t = blockIdx.x;
+    const int tm = m_fast ? t % tiles_m : t / tiles_n, tn = m_fast ? t / tiles_m : t % tiles_n;
+    ffma_tile<S, VA, VB>(p, tm * S::BM, tn * S::BN, sm);
+}
+
+// Many independent SGEMMs: CTA b works on job j with tile0[j] <= b < tile0[j + 1].
+template <class S>
+__global__ void __launch_bounds__(S::NT) ffma_group_kernel(const FfmaJob *__restrict__ jobs, int njobs)
+{
+    extern __shared__ __align__(128) float sm[];
+    const int b = blockIdx.x;
+    int lo = 0, hi = njobs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].tile0 <= b)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const FfmaJob &j = jobs[lo];
+    const int t = b - j.tile0;
+    FfmaArgs p;
+    p.M = j.M; p.N = j.N; p.K = j.K;
+    p.A = j.A; p.lda = j.lda;
+    p.B = j.B; p.ldb = j.ldb;
+    p.C = j.C; p.ldc = j.ldc;
+    p.kblock = 0;
+    const int m0 = (t / j.tiles_n) * S::BM, n0 = (t % j.tiles_n) * S::BN;
+    if (j.vec)
+        ffma_tile<S, true, true>(p, m0, n0, sm);
     else
-        ffma_sgemm_8x8_kernel<false><<<grid, 64, 0, s>>>(a);
+        ffma_tile<S, false, false>(p, m0, n0, sm);
+}
+
+using Big = Shape<128, 128, 16, 8, 16, 3>;
+using Wide = Shape<64, 128, 32, 8, 8, 3>;
+using Square = Shape<64, 64, 32, 4, 8, 3>;
+using Low = Shape<40, 64, 32, 5, 4, 3>;
+using Small = Shape<32, 64, 32, 4, 4, 3>;
+using Tiny = Shape<16, 64, 32, 2, 4, 3>;
+
+// The tile shapes: CTAs resident per SM, and FMA per clock that an SM reaches with
+// one CTA and with all of them (B200; from 256 x 256 x 2048, which gives every shape
+// at most one CTA per SM, and from 1632 x 36548 x 1024).
+struct ShapeInfo {
+    int bm, bn, occ;
+    double one, full;
+};
+constexpr ShapeInfo kShapes[] = {
+    {128, 128, 2, 81.0, 88.4},  // Big: least shared-memory traffic per FMA
+    {64, 128, 3, 78.5, 87.9},   // Wide
+    {64, 64, 4, 61.0, 83.9},    // Square: two or three per SM where Wide leaves SMs idle
+    {40, 64, 4, 48.0, 79.8},    // Low: few rows, and dimensions that 64 pads
+    {32, 64, 4, 43.5, 72.7},    // Small: more CTAs where outputs are few
+    {16, 64, 5, 28.8, 40.0},    // Tiny: at most one CTA per SM
+};
+constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
+
+// Clocks per k that the busiest SM needs for `tiles` tiles of a shape: full waves at
+// the full rate, then the last wave's CTAs per SM, each as fast as alone until the
+// SM saturates. (Occupancy as if every shape's waves were in step; the measured
+// order of the shapes at 14 sizes between 256 x 256 x 2048 and 4096 x 4096 x 2048 is the
+// model's, but for ties.)
+double shape_cost(const ShapeInfo &s, long tiles, int num_sms)
+{
+    const double area = (double)s.bm * s.bn;
+    const long wave = (long)num_sms * s.occ;
+    const long rem = tiles % wave;
+    double t = (double)(tiles / wave) * s.occ * area / s.full;
+    if (rem) {
+        const double c = (double)((rem + num_sms - 1) / num_sms);
+        t += c * area / (c * s.one < s.full ? c * s.one : s.full);
+    }
+    return t;
+}
+
+int pick_shape(long M, long N, int num_sms)
+{
+    int best = 0;
+    double cost = 0.0;
+    for (int i = 0; i < kNumShapes; ++i) {
+        const ShapeInfo &s = kShapes[i];
+        const double c = shape_cost(s, ((M + s.bm - 1) / s.bm) * ((N + s.bn - 1) / s.bn), num_sms);
+        if (i == 0 || c < cost) {
+            best = i;
+            cost = c;
+        }
+    }
+    return best;
+}
+
+// Dynamic shared memory above 48 KB is granted per function and device, once.
+template <class F>
+cudaError_t allow_smem(F *f, int smem, unsigned long long &done, std::mutex &mu)
+{
+    if (smem <= 48 * 1024) return cudaSuccess;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    if (done >> (dev & 63) & 1) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) done |= 1ull << (dev & 63);
+    return e;
+}
+
+template <class S, bool VA, bool VB>
+cudaError_t launch_tiles(const FfmaArgs &a, cudaStream_t s)
+{
+    static unsigned long long done;
+    static std::mutex mu;
+    const cudaError_t e = allow_smem(ffma_sgemm_kernel<S, VA, VB>, S::SMEM, done, mu);
+    if (e != cudaSuccess) return e;
+    const long tm = (a.M + S::BM - 1) / S::BM, tn = (a.N + S::BN - 1) / S::BN;
+    if (tm * tn > 0x7fffffffl) return cudaErrorInvalidConfiguration;
+    ffma_sgemm_kernel<S, VA, VB>
+        <<<(unsigned)(tm * tn), S::NT, S::SMEM, s>>>(a, (int)tm, (int)tn, tm <= tn);
     return cudaGetLastError();
 }
 
-template <int BM, int BN, int BK, int TM, int TN>
-static cudaError_t launch_cfg(const FfmaArgs &a, bool vec, cudaStream_t s)
+template <class S>
+cudaError_t launch_shape(const FfmaArgs &a, cudaStream_t s)
 {
-    dim3 grid((a.N + BN - 1) / BN, (a.M + BM - 1) / BM);
-    dim3 block((BM / TM) * (BN / TN));
-    const bool split = a.kblock > 0 && a.kblock < a.K;
-    if (vec) {
-        if (split)
-            ffma_sgemm_kernel<BM, BN, BK, TM, TN, true, true><<<grid, block, 0, s>>>(a);
-        else
-            ffma_sgemm_kernel<BM, BN, BK, TM, TN, true, false><<<grid, block, 0, s>>>(a);
-    } else {
-        if (split)
-            ffma_sgemm_kernel<BM, BN, BK, TM, TN, false, true><<<grid, block, 0, s>>>(a);
-        else
-            ffma_sgemm_kernel<BM, BN, BK, TM, TN, false, false><<<grid, block, 0, s>>>(a);
-    }
+    const bool va = a.lda % 4 == 0 && ((uintptr_t)a.A & 15) == 0;
+    const bool vb = a.ldb % 4 == 0 && ((uintptr_t)a.B & 15) == 0;
+    if (va) return vb ? launch_tiles<S, true, true>(a, s) : launch_tiles<S, true, false>(a, s);
+    return vb ? launch_tiles<S, false, true>(a, s) : launch_tiles<S, false, false>(a, s);
+}
+
+}  // namespace
+
+int ffma_group_tile(int big) { return big ? Big::BM : Square::BM; }
+
+cudaError_t launch_ffma_group(const FfmaJob *jobs_dev, int njobs, int total_tiles, int big,
+                              cudaStream_t s)
+{
+    static_assert(Big::BM == Big::BN && Square::BM == Square::BN, "jobs are cut into square tiles");
+    static_assert(Big::SMEM <= 48 * 1024 && Square::SMEM <= 48 * 1024, "no attribute needed");
+    if (njobs < 1 || total_tiles < 1) return cudaSuccess;
+    if (big)
+        ffma_group_kernel<Big><<<total_tiles, Big::NT, Big::SMEM, s>>>(jobs_dev, njobs);
+    else
+        ffma_group_kernel<Square><<<total_tiles, Square::NT, Square::SMEM, s>>>(jobs_dev, njobs);
     return cudaGetLastError();
 }
 
 cudaError_t launch_ffma_sgemm(const FfmaArgs &a, int num_sms, cudaStream_t s)
 {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;
-    if (a.kblock > 0 && a.kblock % 16) return cudaErrorInvalidValue;  // K blocks end on slices
-    const bool vec = ((a.lda | a.ldb | a.ldc) % 4 == 0) &&
-                     (((uintptr_t)a.A | (uintptr_t)a.B | (uintptr_t)a.C) % 16 == 0);
-    // FG_FFMA_CFG forces one tile configuration (0..8). By default 128 x 128 x 16
-    // tiles when there are at least two per SM, else 64 x 64 x 16 with 8 x 8 per
-    // thread (measured on B200 with 4 x 8 per thread: 1024^3 25.9 TFLOP/s with
-    // 64 x 64 vs 17.8 with 128 x 128; 4096^3 38.4 with 128 x 128 x 16).
+    if (a.kblock > 0 && a.kblock % 32) return cudaErrorInvalidValue;  // K blocks end on slices
+    // FG_FFMA_CFG forces one row of kShapes
     static const int forced = [] {
         const char *v = getenv("FG_FFMA_CFG");
-        return v ? atoi(v) : -1;
+        const int i = v ? atoi(v) : -1;
+        return i < kNumShapes ? i : -1;
     }();
-    const long t128 = (long)((a.M + 127) / 128) * ((a.N + 127) / 128);
-    const long t12864 = (long)((a.M + 127) / 128) * ((a.N + 63) / 64);
-    int cfg = forced;
-    if (cfg < 0) cfg = t128 >= 2l * num_sms ? 5 : (vec ? 8 : 2);
-    (void)t12864;
-    switch (cfg) {
-    case 8:  // 64 x 64 x 16, 8 x 8 per thread (vector rows and pointers only)
-        if (vec) return launch_8x8(a, s);
-        return launch_cfg<64, 64, 16, 4, 8>(a, vec, s);
-    case 0: return launch_cfg<128, 128, 8, 8, 8>(a, vec, s);   // 256 threads
-    case 1: return launch_cfg<128, 64, 8, 8, 8>(a, vec, s);    // 128 threads
-    case 2: return launch_cfg<64, 64, 16, 4, 8>(a, vec, s);    // 128 threads
-    case 3: return launch_cfg<64, 128, 8, 8, 8>(a, vec, s);    // 128 threads
-    case 4: return launch_cfg<64, 64, 32, 4, 8>(a, vec, s);    // 128 threads
-    case 5: return launch_cfg<128, 128, 16, 8, 8>(a, vec, s);  // 256 threads
-    case 6: return launch_cfg<64, 32, 32, 4, 4>(a, vec, s);    // 128 threads
-    default: return launch_cfg<128, 64, 32, 8, 8>(a, vec, s);  // 128 threads
+    switch (forced >= 0 ? forced : pick_shape(a.M, a.N, num_sms)) {
+    case 0: return launch_shape<Big>(a, s);
+    case 1: return launch_shape<Wide>(a, s);
+    case 2: return launch_shape<Square>(a, s);
+    case 3: return launch_shape<Low>(a, s);
+    case 4: return launch_shape<Small>(a, s);
+    default: return launch_shape<Tiny>(a, s);
     }
 }
 

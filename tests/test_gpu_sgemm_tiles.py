@@ -1,0 +1,50 @@
+"""The plain FP32 SGEMM's tile shapes at the sizes where a tile can go wrong: edges
+in M, N and K, K blocks of 2048 with remainders, rows and pointers that are not
+16-byte aligned, on device memory. Bit for bit the oracle's result (one FMA per k
+in increasing k, K cut into blocks of 2048), NaN and infinity included."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+# the launcher's shape for a 148-SM device beside each size
+SIZES = [
+    (31999, 1000, 17),  # 128 x 128
+    (4096, 4096, 48),   # 64 x 128
+    (1300, 1100, 65),   # 64 x 64
+    (64, 18496, 31),    # 64 x 64, whole tiles
+    (257, 4001, 33),    # 40 x 64
+    (40, 6400, 32),     # 40 x 64, whole tiles
+    (96, 4096, 100),    # 32 x 64
+    (1, 1, 1), (17, 63, 2), (16, 64, 4), (129, 127, 15),  # 16 x 64
+    (35, 457, 2049), (130, 260, 4100), (16, 16, 6144),    # K in blocks of 2048
+]
+
+
+def _device(a, offset):
+    """The array on the device, its first element `offset` floats past an aligned address."""
+    import torch
+    buf = torch.zeros(a.size + offset + 4, device="cuda")
+    t = buf[offset:offset + a.size].view(a.shape)
+    t.copy_(torch.from_numpy(a))
+    return t
+
+
+@pytest.mark.parametrize("offsets", [(0, 0, 0), (1, 0, 0), (0, 2, 3)], ids=["aligned", "a", "bc"])
+@pytest.mark.parametrize("shape", SIZES, ids=["x".join(map(str, s)) for s in SIZES])
+def test_sgemm_tiles_bitexact(shape, offsets):
+    import torch
+    import flashgemm_b200 as fg
+    M, N, K = shape
+    A, B = oracle.sgemm_inputs(M, N, K, seed=M + 3 * N + K)
+    A[M // 2, K - 1] = np.inf   # the last k of a row: a k past it must not meet it
+    B[K - 1, N // 2] = np.nan
+    rows = sorted({0, 1 % M, M // 2, (M - 1) // 3, M - 1}) if M * N > 1 << 20 else list(range(M))
+    want = oracle.sgemm_f32(np.ascontiguousarray(A[rows]), B, kblock=2048)
+    a, b = _device(A, offsets[0]), _device(B, offsets[1])
+    c = _device(np.full((M, N), 7.0, np.float32), offsets[2])
+    fg.sgemm_dev(c, a, b, M, N, K)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(c.cpu().numpy()[rows], want)
