@@ -675,6 +675,7 @@ int run_chain(DevCtx *c, int dtype, int sem, int algo, void *C, long ldc, Mat b,
             f.C = last ? (float *)C : buf[i & 1];
             f.ldc = last ? ldc : ldN;
             f.kblock = 0;  // the multigemm FP32 chain does not split K (kernel_f32.h:3)
+            f.part = nullptr;
             int st = run_kernel(c, FG_PK_FFMA, gemm_flops(M[i], N, K[i]), "ffma stage",
                                 [&] { return launch_ffma_sgemm(f, c->sms, c->work); });
             if (st) return st;
@@ -1170,14 +1171,35 @@ int chain_va(int dtype, void *C, const void *B, long N, int num_gemm, va_list ap
 
 // ---------------------------------------------------------------- SGEMM
 
+// singlegemm blocks K by GEMM_K = 2048 and adds the partial sums into C
+// (singlegemm/src/NN_mp.h:13, :247)
+constexpr int kSgemmKBlock = 2048;
+
+// Workspace of an FFMA SGEMM on stream s. A stream that is being captured gets none:
+// the graph would keep a pointer into the arena, which a later call may grow.
+size_t sgemm_workspace(DevCtx *c, long M, long N, long K, cudaStream_t s)
+{
+    const size_t bytes = ffma_sgemm_workspace(M, N, K, kSgemmKBlock, c->sms);
+    if (!bytes) return 0;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return cap == cudaStreamCaptureStatusNone ? carve_size(bytes) : 0;
+}
+
+// workspace: sgemm_workspace bytes of the arena are reserved for this call
 int run_sgemm(DevCtx *c, int algo, float *C, long ldc, const float *A, long lda, const float *B,
-              long ldb, long M, long N, long K, int kblock)
+              long ldb, long M, long N, long K, size_t workspace)
 {
     if (algo == FG_F32_FFMA) {
         FfmaArgs f;
         f.M = (int)M; f.N = (int)N; f.K = (int)K;
         f.A = A; f.lda = lda; f.B = B; f.ldb = ldb; f.C = C; f.ldc = ldc;
-        f.kblock = kblock;
+        f.kblock = kSgemmKBlock;
+        f.part = workspace ? (float *)arena_take(c, workspace) : nullptr;
+        f.ld_part = round_up(N, 4);
         return run_kernel(c, FG_PK_FFMA, gemm_flops(M, N, K), "ffma sgemm",
                           [&] { return launch_ffma_sgemm(f, c->sms, c->work); });
     }
@@ -1199,9 +1221,12 @@ int host_sgemm(float *C, const float *A, const float *B, long M, long N, long K)
     const long ldk = round_up(K > 0 ? K : 1, 4), ldn = round_up(N, 4);
     size_t need = carve_size((size_t)M * ldk * 4) + carve_size((size_t)K * ldn * 4) +
                   carve_size((size_t)M * ldn * 4) + 4096;
+    size_t workspace = 0;
     if (algo == FG_F32_3XTF32) {
         long Ms[1] = {M}, Ks[1] = {K};
         need += chain_scratch(FG_DT_F32, algo, N, 1, Ms, Ks);
+    } else {
+        need += workspace = sgemm_workspace(c, M, N, K, c->stream);
     }
     if ((st = enter_stream(c, c->stream))) return st;
     if ((st = arena_reserve(c, need))) return st;
@@ -1212,9 +1237,7 @@ int host_sgemm(float *C, const float *A, const float *B, long M, long N, long K)
         CUDA_TRY(copy_rows(ad, ldk * 4, A, K * 4, K * 4, M, cudaMemcpyHostToDevice, c->stream));
         CUDA_TRY(copy_rows(bd, ldn * 4, B, N * 4, N * 4, K, cudaMemcpyHostToDevice, c->stream));
     }
-    // singlegemm blocks K by GEMM_K = 2048 and adds the partial sums into C
-    // (singlegemm/src/NN_mp.h:13, :247)
-    if ((st = run_sgemm(c, algo, cd, ldn, ad, ldk, bd, ldn, M, N, K, 2048))) return st;
+    if ((st = run_sgemm(c, algo, cd, ldn, ad, ldk, bd, ldn, M, N, K, workspace))) return st;
     CUDA_TRY(copy_rows(C, N * 4, cd, ldn * 4, N * 4, M, cudaMemcpyDeviceToHost, c->stream));
     if ((st = collect_status(c))) return st;
     return ok();
@@ -1548,14 +1571,16 @@ FG_EXPORT int fg_sgemm_dev(float *C, const float *A, const float *B, long M, lon
     int st;
     if ((st = get_ctx(&c))) return st;
     std::lock_guard<std::mutex> lk(c->mu);
-    size_t need = 4096;
+    size_t need = 4096, workspace = 0;
     if (algo == FG_F32_3XTF32) {
         long Ms[1] = {M}, Ks[1] = {K};
         need += chain_scratch(FG_DT_F32, algo, N, 1, Ms, Ks);
+    } else {
+        need += workspace = sgemm_workspace(c, M, N, K, user_stream(stream));
     }
     if ((st = enter_stream(c, user_stream(stream)))) return st;
     if ((st = arena_reserve(c, need))) return st;
-    if ((st = run_sgemm(c, algo, C, N, A, K, B, N, M, N, K, 2048))) return st;
+    if ((st = run_sgemm(c, algo, C, N, A, K, B, N, M, N, K, workspace))) return st;
     return ok();
 }
 

@@ -86,18 +86,13 @@ struct Shape {
     static constexpr int STAGE = (BM + BN) * BK;  // floats per ring buffer
     static constexpr int SMEM = ST * STAGE * 4;
     static_assert(BM % TM == 0 && BN % TN == 0 && TN % 4 == 0, "whole fragments");
-    static_assert(BK == 16 || BK == 32, "the swizzle's row length");
+    static_assert(BK == 32, "a row of A's tile is one 128-byte line, its 8 chunks swizzled");
     static_assert(TX == 8 || TX == 16, "a warp holds 4 or 2 rows of column groups");
     static_assert(NT % BK == 0 && NT % (BN / 4) == 0, "copies: a thread's k chunk and column are its own");
 };
 
-// Where the 16-byte chunk c of row r lies in A's tile: BK = 32 rows are one
-// 128-byte line each, BK = 16 rows half a line.
-template <int BK>
-__device__ __forceinline__ int a_chunk(int r, int c)
-{
-    return BK == 16 ? (c ^ ((r >> 1) & 3)) : (c ^ (r & 7));
-}
+// Where the 16-byte chunk c of row r lies in A's tile.
+__device__ __forceinline__ int a_chunk(int r, int c) { return c ^ (r & 7); }
 
 // One BM x BN output tile at (m0, n0). VA / VB: A / B has 16-byte-aligned rows and
 // pointer, and comes in 16-byte copies; else in 4-byte ones. Rows past M read
@@ -122,7 +117,7 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
     const int a_r = tid / A_C, a_c = tid % A_C;
     const int b_r = B_C > NT ? 0 : tid / B_C, b_c = tid % B_C;
     auto a_dst = [&](int r) {
-        return sbase + (r * BK + a_chunk<BK>(r, a_c * EA / 4) * 4 + (EA == 4 ? 0 : a_c % 4)) * 4;
+        return sbase + (r * BK + a_chunk(r, a_c * EA / 4) * 4 + (EA == 4 ? 0 : a_c % 4)) * 4;
     };
     const uint32_t a_dst0 = a_dst(a_r);
     int b_bytes[B_P];
@@ -236,7 +231,7 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
         const float *As = sm + buf * S::STAGE, *Bs = As + BM * BK;
         auto a_quad = [&](int i, int q) {
             const int r = ty + i * TY;
-            return *reinterpret_cast<const float4 *>(&As[r * BK + a_chunk<BK>(r, q) * 4]);
+            return *reinterpret_cast<const float4 *>(&As[r * BK + a_chunk(r, q) * 4]);
         };
         auto b_quad = [&](int k, int j) {
             return *reinterpret_cast<const float4 *>(&Bs[k * BN + tx * 4 + j * 4 * TX]);
@@ -289,7 +284,7 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
 #pragma unroll
                 for (int i = 0; i < TM; ++i) {
                     const int r = ty + i * TY;
-                    const float x = As[r * BK + a_chunk<BK>(r, k / 4) * 4 + (k & 3)];
+                    const float x = As[r * BK + a_chunk(r, k / 4) * 4 + (k & 3)];
                     const unsigned long long ap = pack2(x, x);
 #pragma unroll
                     for (int j = 0; j < TN / 2; ++j) ffma2(acc[i][j], ap, bp[j]);
@@ -305,15 +300,63 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
     }
 }
 
-// m_fast: neighbouring CTAs share columns of B rather than rows of A
+// m_fast: neighbouring CTAs share columns of B rather than rows of A. With p.part,
+// blockIdx.z is a K block of its own: block 0 writes C, block z part z - 1, for
+// ffma_add_blocks_kernel.
 template <class S, bool VA, bool VB>
-__global__ void __launch_bounds__(S::NT) ffma_sgemm_kernel(const FfmaArgs p, int tiles_m, int tiles_n,
+__global__ void __launch_bounds__(S::NT) ffma_sgemm_kernel(FfmaArgs p, int tiles_m, int tiles_n,
                                                            int m_fast)
 {
     extern __shared__ __align__(128) float sm[];
     const int t = blockIdx.x;
     const int tm = m_fast ? t % tiles_m : t / tiles_n, tn = m_fast ? t / tiles_m : t % tiles_n;
+    if (p.part) {
+        const int z = blockIdx.z, k0 = z * p.kblock;
+        p.A += k0;
+        p.B += (size_t)k0 * p.ldb;
+        p.K = min(p.kblock, p.K - k0);
+        if (z > 0) {
+            p.C = p.part + (size_t)(z - 1) * p.M * p.ld_part;
+            p.ldc = p.ld_part;
+        }
+        p.kblock = 0;
+    }
     ffma_tile<S, VA, VB>(p, tm * S::BM, tn * S::BN, sm);
+}
+
+// C = (C + part 0) + part 1 ...: the K blocks' sums, each added in turn as one CTA that
+// runs all blocks of its tile adds them. Four columns of a row per thread; VEC: C's
+// rows are 16-byte aligned (the parts' always are).
+template <bool VEC>
+__global__ void __launch_bounds__(256) ffma_add_blocks_kernel(const FfmaArgs p, int parts)
+{
+    const long quads = (p.N + 3) / 4, total = quads * p.M;
+    const size_t step = (size_t)p.M * p.ld_part;
+    for (long i = blockIdx.x * 256l + threadIdx.x; i < total; i += gridDim.x * 256l) {
+        const long m = i / quads, n = (i - m * quads) * 4;
+        float *c = p.C + m * p.ldc + n;
+        const float *q = p.part + m * p.ld_part + n;
+        float r[4];
+        if (VEC && n + 3 < p.N) {
+            const float4 v = *reinterpret_cast<const float4 *>(c);
+            r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) r[u] = n + u < p.N ? c[u] : 0.f;
+        }
+#pragma unroll 4
+        for (int z = 0; z < parts; ++z) {
+            const float4 v = *reinterpret_cast<const float4 *>(q + z * step);
+            r[0] = r[0] + v.x; r[1] = r[1] + v.y; r[2] = r[2] + v.z; r[3] = r[3] + v.w;
+        }
+        if (VEC && n + 3 < p.N) {
+            *reinterpret_cast<float4 *>(c) = make_float4(r[0], r[1], r[2], r[3]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (n + u < p.N) c[u] = r[u];
+        }
+    }
 }
 
 // Many independent SGEMMs: CTA b works on job j with tile0[j] <= b < tile0[j + 1].
@@ -345,7 +388,6 @@ __global__ void __launch_bounds__(S::NT) ffma_group_kernel(const FfmaJob *__rest
         ffma_tile<S, false, false>(p, m0, n0, sm);
 }
 
-using Big = Shape<128, 128, 16, 8, 16, 3>;
 using Wide = Shape<64, 128, 32, 8, 8, 3>;
 using Square = Shape<64, 64, 32, 4, 8, 3>;
 using Low = Shape<40, 64, 32, 5, 4, 3>;
@@ -360,8 +402,8 @@ struct ShapeInfo {
     double one, full;
 };
 constexpr ShapeInfo kShapes[] = {
-    {128, 128, 2, 81.0, 88.4},  // Big: least shared-memory traffic per FMA
-    {64, 128, 3, 78.5, 87.9},   // Wide
+    {64, 128, 3, 78.5, 87.9},   // Wide: the best rate; 128 x 128 (8 x 16 per thread) gains nothing on
+                                // it and leaves the SMs idle at both ends of a short K
     {64, 64, 4, 61.0, 83.9},    // Square: two or three per SM where Wide leaves SMs idle
     {40, 64, 4, 48.0, 79.8},    // Low: few rows, and dimensions that 64 pads
     {32, 64, 4, 43.5, 72.7},    // Small: more CTAs where outputs are few
@@ -387,19 +429,31 @@ double shape_cost(const ShapeInfo &s, long tiles, int num_sms)
     return t;
 }
 
-int pick_shape(long M, long N, int num_sms)
+// The cheapest shape for `blocks` K blocks side by side (1: none apart), and its cost.
+int pick_shape(long M, long N, double blocks, int num_sms, double &cost)
 {
     int best = 0;
-    double cost = 0.0;
     for (int i = 0; i < kNumShapes; ++i) {
         const ShapeInfo &s = kShapes[i];
-        const double c = shape_cost(s, ((M + s.bm - 1) / s.bm) * ((N + s.bn - 1) / s.bn), num_sms);
+        const double tiles = (double)((M + s.bm - 1) / s.bm) * ((N + s.bn - 1) / s.bn);
+        const double c = shape_cost(s, (long)(tiles * blocks + 0.999), num_sms);
         if (i == 0 || c < cost) {
             best = i;
             cost = c;
         }
     }
     return best;
+}
+
+// FG_FFMA_CFG forces one row of kShapes
+int forced_shape()
+{
+    static const int forced = [] {
+        const char *v = getenv("FG_FFMA_CFG");
+        const int i = v ? atoi(v) : -1;
+        return i < kNumShapes ? i : -1;
+    }();
+    return forced;
 }
 
 // Dynamic shared memory above 48 KB is granted per function and device, once.
@@ -425,8 +479,9 @@ cudaError_t launch_tiles(const FfmaArgs &a, cudaStream_t s)
     if (e != cudaSuccess) return e;
     const long tm = (a.M + S::BM - 1) / S::BM, tn = (a.N + S::BN - 1) / S::BN;
     if (tm * tn > 0x7fffffffl) return cudaErrorInvalidConfiguration;
+    const unsigned blocks = a.part ? (unsigned)((a.K + a.kblock - 1) / a.kblock) : 1u;
     ffma_sgemm_kernel<S, VA, VB>
-        <<<(unsigned)(tm * tn), S::NT, S::SMEM, s>>>(a, (int)tm, (int)tn, tm <= tn);
+        <<<dim3((unsigned)(tm * tn), 1, blocks), S::NT, S::SMEM, s>>>(a, (int)tm, (int)tn, tm <= tn);
     return cudaGetLastError();
 }
 
@@ -441,39 +496,77 @@ cudaError_t launch_shape(const FfmaArgs &a, cudaStream_t s)
 
 }  // namespace
 
-int ffma_group_tile(int big) { return big ? Big::BM : Square::BM; }
+void ffma_group_tile(int big, int &tile_m, int &tile_n)
+{
+    tile_m = big ? Wide::BM : Square::BM;
+    tile_n = big ? Wide::BN : Square::BN;
+}
 
 cudaError_t launch_ffma_group(const FfmaJob *jobs_dev, int njobs, int total_tiles, int big,
                               cudaStream_t s)
 {
-    static_assert(Big::BM == Big::BN && Square::BM == Square::BN, "jobs are cut into square tiles");
-    static_assert(Big::SMEM <= 48 * 1024 && Square::SMEM <= 48 * 1024, "no attribute needed");
     if (njobs < 1 || total_tiles < 1) return cudaSuccess;
-    if (big)
-        ffma_group_kernel<Big><<<total_tiles, Big::NT, Big::SMEM, s>>>(jobs_dev, njobs);
-    else
+    static unsigned long long done[2];
+    static std::mutex mu;
+    if (big) {
+        const cudaError_t e = allow_smem(ffma_group_kernel<Wide>, Wide::SMEM, done[0], mu);
+        if (e != cudaSuccess) return e;
+        ffma_group_kernel<Wide><<<total_tiles, Wide::NT, Wide::SMEM, s>>>(jobs_dev, njobs);
+    } else {
+        const cudaError_t e = allow_smem(ffma_group_kernel<Square>, Square::SMEM, done[1], mu);
+        if (e != cudaSuccess) return e;
         ffma_group_kernel<Square><<<total_tiles, Square::NT, Square::SMEM, s>>>(jobs_dev, njobs);
+    }
     return cudaGetLastError();
+}
+
+// K blocks are independent sums until they are added, so where the tiles alone leave
+// SMs idle they run side by side, the sums of all but the first in a workspace, and
+// a second kernel adds them in order: the same bits. That costs the launch (about
+// 3 us) and the parts' traffic; it is taken where the tiles' cost falls by more.
+// Measured (B200, us a call; first figure: this tile, blocks in turn): 35 x 8457 x 2560
+// 99 -> 92, 128 x 2048 x 4096 98 -> 76 (the kernel before this tile: 278),
+// 1024 x 16 x 500000 1468 (38000 before).
+size_t ffma_sgemm_workspace(long M, long N, long K, int kblock, int num_sms)
+{
+    if (M <= 0 || N <= 0 || kblock <= 0 || K <= kblock) return 0;
+    const long blocks = (K + kblock - 1) / kblock;
+    if (blocks > 65535) return 0;
+    const long ld = (N + 3) / 4 * 4;
+    const double part_bytes = (double)(blocks - 1) * M * ld * 4;
+    if (part_bytes > (double)(1l << 30)) return 0;  // such results fill the SMs anyhow
+    double whole = 0.0, apart = 0.0;
+    pick_shape(M, N, 1.0, num_sms, whole);
+    pick_shape(M, N, (double)K / kblock, num_sms, apart);
+    // clocks: 6000 for the launch, the parts written and read once at 3000 bytes a clock
+    return apart * kblock + 6000.0 + 2.0 * part_bytes / 3000.0 < whole * K ? (size_t)part_bytes : 0;
 }
 
 cudaError_t launch_ffma_sgemm(const FfmaArgs &a, int num_sms, cudaStream_t s)
 {
     if (a.M <= 0 || a.N <= 0) return cudaSuccess;
     if (a.kblock > 0 && a.kblock % 32) return cudaErrorInvalidValue;  // K blocks end on slices
-    // FG_FFMA_CFG forces one row of kShapes
-    static const int forced = [] {
-        const char *v = getenv("FG_FFMA_CFG");
-        const int i = v ? atoi(v) : -1;
-        return i < kNumShapes ? i : -1;
-    }();
-    switch (forced >= 0 ? forced : pick_shape(a.M, a.N, num_sms)) {
-    case 0: return launch_shape<Big>(a, s);
-    case 1: return launch_shape<Wide>(a, s);
-    case 2: return launch_shape<Square>(a, s);
-    case 3: return launch_shape<Low>(a, s);
-    case 4: return launch_shape<Small>(a, s);
-    default: return launch_shape<Tiny>(a, s);
+    double cost = 0.0;
+    const int shape = forced_shape() >= 0 ? forced_shape()
+                                          : pick_shape(a.M, a.N, a.part ? (double)a.K / a.kblock : 1.0,
+                                                       num_sms, cost);
+    cudaError_t e;
+    switch (shape) {
+    case 0: e = launch_shape<Wide>(a, s); break;
+    case 1: e = launch_shape<Square>(a, s); break;
+    case 2: e = launch_shape<Low>(a, s); break;
+    case 3: e = launch_shape<Small>(a, s); break;
+    default: e = launch_shape<Tiny>(a, s); break;
     }
+    if (e != cudaSuccess || !a.part) return e;
+    const int parts = (a.K + a.kblock - 1) / a.kblock - 1;
+    const long ctas = ((a.N + 3) / 4 * (long)a.M + 255) / 256;
+    const unsigned grid = (unsigned)(ctas < num_sms * 8l ? ctas : num_sms * 8l);
+    if (a.ldc % 4 == 0 && ((uintptr_t)a.C & 15) == 0)
+        ffma_add_blocks_kernel<true><<<grid, 256, 0, s>>>(a, parts);
+    else
+        ffma_add_blocks_kernel<false><<<grid, 256, 0, s>>>(a, parts);
+    return cudaGetLastError();
 }
 
 }  // namespace fg

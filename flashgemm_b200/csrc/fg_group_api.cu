@@ -393,12 +393,13 @@ int group_build(DevCtx *c, int dtype, int algo, int kernel, int order, int nchai
             long t128 = 0;
             for (auto &f : lv.jobs) t128 += (long)((f.M + 127) / 128) * ((f.N + 127) / 128);
             lv.big = t128 >= 2l * c->sms ? 1 : 0;
-            const int tile = ffma_group_tile(lv.big);
+            int tile_m, tile_n;
+            ffma_group_tile(lv.big, tile_m, tile_n);
             long t = 0;
             for (auto &f : lv.jobs) {
                 f.tile0 = (int)t;
-                f.tiles_n = (f.N + tile - 1) / tile;
-                t += (long)((f.M + tile - 1) / tile) * f.tiles_n;
+                f.tiles_n = (f.N + tile_n - 1) / tile_n;
+                t += (long)((f.M + tile_m - 1) / tile_m) * f.tiles_n;
             }
             if (t > (1l << 31) - 1) return fail(FG_ERR_INVALID, "group too large");
             lv.tiles = (int)t;

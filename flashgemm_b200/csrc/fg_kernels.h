@@ -294,8 +294,15 @@ struct FfmaArgs {
     const float *B; long ldb;
     float *C; long ldc;
     int kblock;
+    // optional (else null): ffma_sgemm_workspace bytes, in which K blocks that run side by
+    // side leave their sums (M rows of ld_part >= N floats, a multiple of 4, per block)
+    float *part;
+    long ld_part;
 };
 cudaError_t launch_ffma_sgemm(const FfmaArgs &a, int num_sms, cudaStream_t s);
+// Bytes of workspace with which this SGEMM runs its K blocks side by side (ld_part: N
+// rounded up to 4); 0 where it does not.
+size_t ffma_sgemm_workspace(long M, long N, long K, int kblock, int num_sms);
 
 // FP32 -> (hi, lo) TF32 split of a rows x cols matrix (leading dims ld_in / ld_out).
 cudaError_t launch_split_tf32(const float *in, long ld_in, float *hi, float *lo, long ld_out,
@@ -329,7 +336,8 @@ struct FfmaJob {
     int tiles_n; // column tiles of this job
     int vec;     // 16-byte-aligned rows and pointers
 };
-int ffma_group_tile(int big);  // tile edge of the grouped FFMA kernel (64, or 128 when big)
+// Tiles of the grouped FFMA kernel (64 x 64, or 64 x 128 when big).
+void ffma_group_tile(int big, int &tile_m, int &tile_n);
 cudaError_t launch_ffma_group(const FfmaJob *jobs_dev, int njobs, int total_tiles, int big,
                               cudaStream_t s);
 

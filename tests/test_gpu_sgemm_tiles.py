@@ -11,15 +11,15 @@ pytestmark = pytest.mark.gpu
 
 # the launcher's shape for a 148-SM device beside each size
 SIZES = [
-    (31999, 1000, 17),  # 128 x 128
-    (4096, 4096, 48),   # 64 x 128
+    (31999, 1000, 17), (4096, 4096, 48),  # 64 x 128
     (1300, 1100, 65),   # 64 x 64
     (64, 18496, 31),    # 64 x 64, whole tiles
     (257, 4001, 33),    # 40 x 64
     (40, 6400, 32),     # 40 x 64, whole tiles
     (96, 4096, 100),    # 32 x 64
     (1, 1, 1), (17, 63, 2), (16, 64, 4), (129, 127, 15),  # 16 x 64
-    (35, 457, 2049), (130, 260, 4100), (16, 16, 6144),    # K in blocks of 2048
+    (35, 457, 2049), (130, 260, 4100), (16, 16, 6144),    # K in blocks of 2048, side by side
+    (1300, 1100, 2080),                                   # and in turn
 ]
 
 
