@@ -30,6 +30,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "fg_tc_common.cuh"
@@ -307,6 +308,12 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
             uint32_t rph = 0;
             unsigned tiles = 0;      // tiles issued: accumulator tiles % kNAcc, phase (tiles / kNAcc) & 1
             uint32_t xr = 0;         // bit s: the xready phase to wait for on buffer s
+            // descriptors of ring slot 0's first weight box and activation boxes, and
+            // of operand buffer 0
+            const uint64_t a_desc0 = smem_desc(smem_u32(ring), 16, 1024, SMEM_SW128);
+            const uint64_t b_desc0 =
+                smem_desc(smem_u32(ring) + g.ra * kNABytes, G::BOX_BYTES, 1024, SMEM_SW128);
+            const uint64_t x_desc0 = smem_desc(smem_u32(xbuf), 16, 1024, SMEM_SW128);
             int slot, j, st, r0, nt;
             for (int u = 0; walk.next(slot, j, st, r0, nt); ++u) {
                 const NarrowStage &cs = g.st[st];
@@ -331,37 +338,41 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
                 tc_fence_after();
                 if (g.trace) ntrace(g, u, NT_MMA_START, globaltimer_ns());
                 const int nkb = (cs.K + G::BK - 1) / G::BK;
-                const uint32_t xb = smem_u32(xbuf + slot * g.x_bytes);
-                for (int kb = 0; kb < nkb; ++kb) {
-                    if (!mbar_wait(&bars->wfull[r], rph, status, KERR_WAIT_FULL)) {
-                        n_set_abort(bars);
-                        goto mma_done;
-                    }
-                    tc_fence_after();
-                    const uint32_t s_addr = smem_u32(ring + r * g.slot_bytes);
-                    for (int t = 0; t < nt; ++t) {
-                        const uint32_t d_tmem = tmem_base + ((tiles + t) % kNAcc) * kNBN;
-                        const uint32_t a_addr = s_addr + t * kNABytes;
+                // The issue loop carries no descriptor arithmetic but additions to the
+                // bases built before it (field: bytes >> 4), its operand kind fixed: an
+                // MMA here takes 64 clocks of the tensor pipe, and encoding both
+                // descriptors anew for each one took the issuing thread longer.
+                auto issue = [&](auto first_tag) -> bool {
+                    constexpr bool first = decltype(first_tag)::value;
+                    constexpr uint32_t idesc = first ? G::idesc_mn : G::idesc_k;
+                    constexpr uint64_t b_step = (first ? G::B_KSTEP : 32) >> 4;
+                    const uint64_t x0 = x_desc0 + (uint64_t)((slot * g.x_bytes) >> 4);
+                    uint32_t acc = 0;
+                    for (int kb = 0; kb < nkb; ++kb) {
+                        if (!mbar_wait(&bars->wfull[r], rph, status, KERR_WAIT_FULL)) return false;
+                        tc_fence_after();
+                        const uint64_t slot_off = (uint64_t)((r * g.slot_bytes) >> 4);
+                        const uint64_t bd = first ? b_desc0 + slot_off : x0 + (uint64_t)(kb * (kNKbBytes >> 4));
+                        uint64_t ad = a_desc0 + slot_off;
+                        for (int t = 0; t < nt; ++t, ad += kNABytes >> 4) {
+                            const uint32_t d_tmem = tmem_base + ((tiles + t) % kNAcc) * kNBN;
+                            tc_mma<KIND>(d_tmem, ad, bd, idesc, acc);
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const uint64_t ad = smem_desc(a_addr + k * 32, 16, 1024, SMEM_SW128);
-                            if (st == 0) {
-                                const uint64_t bd =
-                                    smem_desc(s_addr + g.ra * kNABytes + k * G::B_KSTEP,
-                                              G::BOX_BYTES, 1024, SMEM_SW128);
-                                tc_mma<KIND>(d_tmem, ad, bd, G::idesc_mn, (kb | k) != 0);
-                            } else {
-                                const uint64_t bd =
-                                    smem_desc(xb + kb * kNKbBytes + k * 32, 16, 1024, SMEM_SW128);
-                                tc_mma<KIND>(d_tmem, ad, bd, G::idesc_k, (kb | k) != 0);
-                            }
+                            for (int k = 1; k < 4; ++k)
+                                tc_mma<KIND>(d_tmem, ad + k * 2, bd + k * b_step, idesc, 1);
+                        }
+                        acc = 1;
+                        tc_commit(&bars->wempty[r]);
+                        if (++r == RING) {
+                            r = 0;
+                            rph ^= 1;
                         }
                     }
-                    tc_commit(&bars->wempty[r]);
-                    if (++r == RING) {
-                        r = 0;
-                        rph ^= 1;
-                    }
+                    return true;
+                };
+                if (!(st == 0 ? issue(std::true_type{}) : issue(std::false_type{}))) {
+                    n_set_abort(bars);
+                    goto mma_done;
                 }
                 for (int t = 0; t < nt; ++t) tc_commit(&bars->acc_full[(tiles + t) % kNAcc]);
                 tiles += nt;
