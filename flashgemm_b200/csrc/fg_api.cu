@@ -693,6 +693,14 @@ int run_chain(DevCtx *c, int dtype, int sem, int algo, void *C, long ldc, Mat b,
     if (dtype == FG_DT_F32) {  // 3xTF32
         std::vector<const float *> wh(n), wl(n);
         std::vector<long> wld(n);
+        SplitBatch batch;
+        auto split = [&]() -> int {
+            if (!batch.n) return FG_OK;
+            const int st = run_kernel(c, FG_PK_AUX, 0.0, "tf32 split",
+                                      [&] { return launch_split_tf32(batch, c->work); });
+            batch.n = 0;
+            return st;
+        };
         for (int i = 0; i < n; ++i) {
             const long ldk = round_up(K[i], 4);
             wld[i] = ldk;
@@ -706,16 +714,18 @@ int run_chain(DevCtx *c, int dtype, int sem, int algo, void *C, long ldc, Mat b,
             float *l = (float *)arena_take(c, (size_t)M[i] * ldk * 4);
             wh[i] = h;
             wl[i] = l;
-            int st = run_kernel(c, FG_PK_AUX, 0.0, "tf32 split (weights)", [&] {
-                return launch_split_tf32((const float *)a[i].p, a[i].ld, h, l, ldk, M[i], K[i],
-                                         c->work);
-            });
-            if (st) return st;
+            if (batch.n == kSplitBatch)
+                if (int st = split()) return st;
+            batch.job[batch.n++] = SplitJob{(const float *)a[i].p, a[i].ld, h, l, ldk, M[i], K[i]};
         }
-        if (fused_enabled() && panel_enabled() && panel_eligible(N, n, M, K) &&
-            aligned16(b.p) && aligned16(C) && b.ld % 4 == 0 && ldc % 4 == 0) {
-            // every dimension fits on chip: one launch, intermediates in shared memory
-            PanelChainArgs pa;
+        const bool b16 = aligned16(b.p) && b.ld % 4 == 0;
+        const bool panel = fused_enabled() && b16 && aligned16(C) && ldc % 4 == 0 && panel_enabled() &&
+                           panel_eligible(N, n, M, K);
+        const bool column = !panel && fused_enabled() && b16 && column_preferred(N, n, M, K, c->sms);
+        if (panel || column)
+            if (int st = split()) return st;  // the weights; B is split on the way in
+        PanelChainArgs pa;
+        if (panel || column) {
             memset(&pa, 0, sizeof pa);
             pa.n = n;
             pa.N = N;
@@ -731,6 +741,23 @@ int run_chain(DevCtx *c, int dtype, int sem, int algo, void *C, long ldc, Mat b,
                 pa.K[i] = K[i];
                 pa.kchunk[i] = tf32_chunk_blocks(K[i]);
             }
+        }
+        if (column) {
+            // intermediates in tensor memory, B read once; operands whose rows the tensor
+            // maps cannot describe fall through to one launch per stage
+            double fl = 0.0;
+            for (int i = 0; i < n; ++i) fl += gemm_flops(M[i], N, K[i]);
+            cudaError_t le = cudaSuccess;
+            const int st = run_kernel(c, FG_PK_TC_TF32X3, fl, "column chain", [&] {
+                le = launch_column(pa, c->sms, c->status, c->work);
+                return le;
+            });
+            if (le != cudaErrorNotSupported) return st;
+            g_launches.fetch_sub(1, std::memory_order_relaxed);
+            ok();
+        }
+        if (panel) {
+            // every dimension fits on chip: one launch, intermediates in shared memory
             double fl = 0.0;
             for (int i = 0; i < n; ++i) fl += gemm_flops(M[i], N, K[i]);
             const long nblocks = (N + 127) / 128;
@@ -771,9 +798,10 @@ int run_chain(DevCtx *c, int dtype, int sem, int algo, void *C, long ldc, Mat b,
         }
         float *xh = (float *)arena_take(c, (size_t)K[0] * ldN * 4);
         float *xl = (float *)arena_take(c, (size_t)K[0] * ldN * 4);
-        int st = run_kernel(c, FG_PK_AUX, 0.0, "tf32 split (activations)", [&] {
-            return launch_split_tf32((const float *)b.p, b.ld, xh, xl, ldN, K[0], N, c->work);
-        });
+        if (batch.n == kSplitBatch)
+            if (int st = split()) return st;
+        batch.job[batch.n++] = SplitJob{(const float *)b.p, b.ld, xh, xl, ldN, K[0], N};
+        int st = split();
         if (st) return st;
         float *ph[2] = {nullptr, nullptr}, *pl[2] = {nullptr, nullptr};
         if (n > 1)
@@ -1342,9 +1370,9 @@ int register_weights(int dtype, const void *A, long M, long K, int where, fg_wei
             free_weights(w);
             return st;
         }
-        if ((st = launch(launch_split_tf32((const float *)w->main, w->ld, w->hi, w->lo, w->ld, M,
-                                           K, c->stream),
-                         "tf32 split (registered weights)"))) {
+        SplitBatch batch;
+        batch.job[batch.n++] = SplitJob{(const float *)w->main, w->ld, w->hi, w->lo, w->ld, M, K};
+        if ((st = launch(launch_split_tf32(batch, c->stream), "tf32 split (registered weights)"))) {
             free_weights(w);
             return st;
         }

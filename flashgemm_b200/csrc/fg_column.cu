@@ -1,0 +1,572 @@
+// FP32 (3xTF32) chains with narrow intermediates, kept in tensor memory: the
+// column chain.
+//
+// The reference runs all stages of a 32-column panel back to back on one core
+// and writes each stage's output straight into the next stage's packed operand
+// (multigemm/src/flashgemm.c:123-148; kernel_f32.h:470), so its intermediates
+// never leave the core. Its own test chains are wide and narrow: N up to 65536
+// activation columns, K_1 up to 8400, intermediates of 16 to 336 rows
+// (multigemm/test/test_f32_3.c:14-48). Here one CTA runs a 128-column block of
+// such a chain from B to C.
+//
+// Each stage computes the transposed product D^T = X^T W^T: the block's 128
+// columns are the MMA's M, the stage's rows (padded to 16) its N. Both D and the A
+// operand X^T live in tensor memory, where lane n is column n of the block and a
+// TMEM column is one row of the stage (D) or one k (A). So the result of a stage
+// lies exactly as the next stage's operand has to: an epilogue thread reads its
+// column's sums, splits them into the TF32 pair (hi, lo) and writes them back as the
+// next A, with no shared memory, no swizzle and no proxy fence between. The first
+// stage's operand comes the same way: B lands by TMA as plain FP32, four splitter
+// warps read it (a thread its own column, conflict-free) and put (hi, lo) into a ring
+// of 16-deep granules in TMEM. Only the weights are shared-memory operands.
+//
+// What bounds it: the tensor pipe (three TF32 MMAs per 8 k, 48 clocks each up to 96
+// rows, rows / 2 above) and, on many columns, reading B once. The launch-per-stage
+// path that it replaces wrote B's split to memory and read it back (3x its bytes)
+// and paid a launch and a memory round trip per stage. Measured (B200, us a call, that
+// path -> this): SPLICE_NUMBERS
+//
+// The arithmetic is that path's: per 8 k the correction terms lo * hi, then hi * lo,
+// into their own accumulator and hi * hi into the chunk's; every `kchunk` k-blocks
+// of 32 the chunk's sum goes to FP32 registers, the correction is added once at the
+// end; so the results are the same bits.
+//
+// Warp 0 is the TMA producer, warp 1 allocates TMEM and issues MMAs, warps 2-5 split,
+// warps 6-9 run the epilogues (a warp of each group per TMEM lane quarter). Accumulators
+// are [d0 | c | d1]: two chunk sums around the correction. TMEM from the bottom: stage
+// 0's accumulators, or a later stage's A operand and then its accumulators (dead and
+// live parts never meet: every MMA of a stage has completed, and a lane has read its
+// sums, before that lane's operand is written); the granule ring above all of them, so
+// that the next block's input is split while this block's last stages run. Every wait
+// is bounded (fg_ptx.cuh); no CTA waits on another.
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstring>
+#include <memory>
+#include <mutex>
+#include <vector>
+
+#include "fg_tc_common.cuh"
+
+namespace fg {
+
+namespace {
+
+constexpr int kCBN = 128;                     // columns per block (MMA M)
+constexpr int kCBK = 32;                      // k per k-block (a 128-byte weight row)
+constexpr int kCXBytes = kCBN * kCBK * 4;     // a k-block of B: 32 rows of 128 floats
+constexpr int kCGran = 16;                    // k per granule of the A ring
+constexpr int kCGranCols = 2 * kCGran;        // its TMEM columns: hi, then lo
+constexpr int kCThreads = 320;
+constexpr int kCMaxRing = 8, kCMaxGran = 8;
+constexpr int kCFixed = 512 + 1024;           // barriers, alignment
+constexpr int kCMaxSmem = 232448;
+constexpr int kCHalfSmem = 113 * 1024;        // two CTAs per SM
+// Two builds: up to 48 rows per tile (half of TMEM and of shared memory, two CTAs per
+// SM, so that one CTA's chain of stages fills the other's waits) and up to 144
+constexpr int kCSmallRows = 48, kCRows = 144;
+
+struct ColStage {
+    CUtensorMap tm_hi, tm_lo;  // weights, K-major boxes of `rows` rows x 128 bytes
+    int M, K, kchunk;
+    int rows, tiles;           // rows per tile (a multiple of 16); more than one tile: last stage only
+    int acc;                   // TMEM column of its accumulators
+};
+
+struct alignas(64) ColArgs {
+    CUtensorMap tm_x;          // B: boxes of 128 columns x 32 rows, no swizzle
+    ColStage st[kPanelMaxStages];
+    float *C;
+    long ldc;
+    int n, N, nblocks;
+    int ring, slot_bytes;      // shared-memory ring: B's k-block, then hi and lo weight boxes
+    int gran, gran0;           // A ring: granules, first TMEM column
+    int tmem_cols, smem, small;
+    int *status;
+};
+
+struct __align__(8) ColBars {
+    uint64_t full[kCMaxRing];                      // shared-memory ring: TMA bytes
+    uint64_t empty[kCMaxRing];                     // MMAs retired, and the 4 splitter warps are past it
+    uint64_t afull[kCMaxGran], aempty[kCMaxGran];  // A ring (4 splitter warps / MMAs retired)
+    uint64_t dfull[2], dempty[2];                  // chunk sums (MMAs retired / 4 epilogue warps)
+    uint64_t cfull;                                // a tile's MMAs have all retired
+    uint64_t drained;                              // the epilogue warps have read all of the tile
+    uint64_t xready;                               // the next stage's A operand is in place
+    uint64_t mma_done;
+    uint32_t tmem_base;
+    int abort;
+};
+static_assert(sizeof(ColBars) <= 512, "barrier block");
+
+__device__ __forceinline__ void c_set_abort(ColBars *b) { *reinterpret_cast<volatile int *>(&b->abort) = 1; }
+__device__ __forceinline__ bool c_aborted(ColBars *b) { return *reinterpret_cast<volatile int *>(&b->abort) != 0; }
+
+// A position in a ring and the parity of its current round.
+struct RingPos {
+    int i = 0;
+    uint32_t ph = 0;
+    __device__ __forceinline__ void next(int n)
+    {
+        if (++i == n) {
+            i = 0;
+            ph ^= 1;
+        }
+    }
+};
+
+}  // namespace
+
+// NC: 16-row groups of the widest tile; PER: CTAs per SM
+template <int NC, int PER>
+__global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_constant__ ColArgs g)
+{
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    uint8_t *smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+    ColBars *bars = reinterpret_cast<ColBars *>(smem + g.ring * g.slot_bytes);
+    int *status = g.status;
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int r = 0; r < kCMaxRing; ++r) {
+            mbar_init(&bars->full[r], 1);
+            mbar_init(&bars->empty[r], 5);
+        }
+        for (int r = 0; r < kCMaxGran; ++r) {
+            mbar_init(&bars->afull[r], 4);
+            mbar_init(&bars->aempty[r], 1);
+        }
+        for (int d = 0; d < 2; ++d) {
+            mbar_init(&bars->dfull[d], 1);
+            mbar_init(&bars->dempty[d], 4);
+        }
+        mbar_init(&bars->cfull, 1);
+        mbar_init(&bars->drained, 4);
+        mbar_init(&bars->xready, 4);
+        mbar_init(&bars->mma_done, 1);
+        bars->abort = 0;
+        fence_mbar_init();
+        tma_prefetch_desc(&g.tm_x);
+        for (int i = 0; i < g.n; ++i) {
+            tma_prefetch_desc(&g.st[i].tm_hi);
+            tma_prefetch_desc(&g.st[i].tm_lo);
+        }
+    }
+    if (warp == 1) tmem_alloc(&bars->tmem_base, g.tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = bars->tmem_base;
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ TMA producer
+        if (lane == 0) {
+            RingPos s;
+            uint32_t pending = 0, pending_ph = 0;
+            for (int blk = blockIdx.x; blk < g.nblocks; blk += gridDim.x) {
+                for (int st = 0; st < g.n; ++st) {
+                    const ColStage &cs = g.st[st];
+                    const int nkb = (cs.K + kCBK - 1) / kCBK;
+                    const int w_bytes = cs.rows * 128;
+                    const uint32_t tx = 2u * w_bytes + (st == 0 ? kCXBytes : 0);
+                    for (int t = 0; t < cs.tiles; ++t)
+                        for (int kb = 0; kb < nkb; ++kb) {
+                            if (!mbar_wait(&bars->empty[s.i], s.ph ^ 1, status, KERR_WAIT_EMPTY)) {
+                                c_set_abort(bars);
+                                goto producer_done;
+                            }
+                            uint8_t *p = smem + s.i * g.slot_bytes;
+                            mbar_arrive_expect_tx(&bars->full[s.i], tx);
+                            if (st == 0) tma_load_2d(p, &g.tm_x, &bars->full[s.i], blk * kCBN, kb * kCBK);
+                            tma_load_2d(p + kCXBytes, &cs.tm_hi, &bars->full[s.i], kb * kCBK, t * cs.rows);
+                            tma_load_2d(p + kCXBytes + w_bytes, &cs.tm_lo, &bars->full[s.i], kb * kCBK,
+                                        t * cs.rows);
+                            pending |= 1u << s.i;
+                            pending_ph = (pending_ph & ~(1u << s.i)) | (s.ph << s.i);
+                            s.next(g.ring);
+                        }
+                }
+                if (c_aborted(bars)) break;
+            }
+        producer_done:
+            // never leave with copies in flight into this CTA's shared memory
+            for (int i = 0; i < g.ring; ++i)
+                if (pending & (1u << i))
+                    mbar_wait(&bars->full[i], (pending_ph >> i) & 1u, status, KERR_WAIT_FULL);
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer
+        if (lane == 0) {
+            RingPos s, a;
+            uint32_t chunks = 0;  // chunk sums started: buffer chunks & 1, round chunks >> 1
+            uint32_t tiles = 0, xr = 0;
+            const uint64_t w_desc0 = smem_desc(smem_u32(smem) + kCXBytes, 16, 1024, SMEM_SW128);
+            bool ok = true;
+            for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
+                for (int st = 0; ok && st < g.n; ++st) {
+                    const ColStage &cs = g.st[st];
+                    const int nkb = (cs.K + kCBK - 1) / kCBK;
+                    const int kchunk = cs.kchunk > 0 ? cs.kchunk : nkb;
+                    const uint32_t idesc = make_idesc(1, 2, 2, 0, 0, kCBN, cs.rows);
+                    const uint64_t lo_off = (uint64_t)((cs.rows * 128) >> 4);
+                    const uint32_t acc = tmem_base + cs.acc, c_tmem = acc + cs.rows;
+                    // a later stage's A: hi at column 0, lo after the previous stage's padded rows
+                    const uint32_t x_lo = st > 0 ? (uint32_t)g.st[st - 1].rows : 0u;
+                    if (st > 0) {
+                        ok = mbar_wait(&bars->xready, xr & 1u, status, KERR_WAIT_FULL);
+                        ++xr;
+                    }
+                    for (int t = 0; ok && t < cs.tiles; ++t, ++tiles) {
+                        // the accumulators (and what overlies them) are free once the tile before is read
+                        if (!(ok = mbar_wait(&bars->drained, (tiles & 1u) ^ 1u, status, KERR_WAIT_ACC_EMPTY)))
+                            break;
+                        uint32_t more_c = 0, more_d = 0, d_tmem = acc;
+                        int left = 0;  // k-blocks left of the chunk
+                        for (int kb = 0; kb < nkb; ++kb) {
+                            if (left == 0) {
+                                const uint32_t b = chunks & 1u;
+                                if (!(ok = mbar_wait(&bars->dempty[b], ((chunks >> 1) & 1u) ^ 1u, status,
+                                                     KERR_WAIT_ACC_EMPTY)))
+                                    break;
+                                d_tmem = acc + (b ? 2 * cs.rows : 0);
+                                more_d = 0;
+                                left = kchunk;
+                            }
+                            if (!(ok = mbar_wait(&bars->full[s.i], s.ph, status, KERR_WAIT_FULL))) break;
+                            tc_fence_after();
+                            const uint64_t w = w_desc0 + (uint64_t)((s.i * g.slot_bytes) >> 4);
+                            const int steps = min(4, (cs.K - kb * kCBK + 7) / 8);  // 8 k each
+                            auto step = [&](uint32_t hi, uint32_t lo, int k) {
+                                const uint64_t wk = w + (uint64_t)(k * 2);
+                                tc_mma_ts_tf32(c_tmem, lo, wk, idesc, more_c);
+                                tc_mma_ts_tf32(c_tmem, hi, wk + lo_off, idesc, 1);
+                                tc_mma_ts_tf32(d_tmem, hi, wk, idesc, more_d);
+                                more_c = more_d = 1;
+                            };
+                            if (st == 0) {
+                                for (int k0 = 0; k0 < steps; k0 += 2) {
+                                    if (!(ok = mbar_wait(&bars->afull[a.i], a.ph, status, KERR_WAIT_FULL))) break;
+                                    tc_fence_after();
+                                    const uint32_t x = tmem_base + g.gran0 + a.i * kCGranCols;
+                                    step(x, x + kCGran, k0);
+                                    if (k0 + 1 < steps) step(x + 8, x + kCGran + 8, k0 + 1);
+                                    tc_commit(&bars->aempty[a.i]);
+                                    a.next(g.gran);
+                                }
+                                if (!ok) break;
+                            } else {
+                                const uint32_t x = tmem_base + kb * kCBK;
+                                for (int k = 0; k < steps; ++k) step(x + 8 * k, x + x_lo + 8 * k, k);
+                            }
+                            tc_commit(&bars->empty[s.i]);
+                            s.next(g.ring);
+                            if (--left == 0 || kb + 1 == nkb) {
+                                tc_commit(&bars->dfull[chunks & 1u]);
+                                ++chunks;
+                                left = 0;
+                            }
+                        }
+                        if (!ok) break;
+                        tc_commit(&bars->cfull);
+                    }
+                }
+                if (c_aborted(bars)) break;
+            }
+            if (!ok) c_set_abort(bars);
+            tc_commit(&bars->mma_done);
+            mbar_wait(&bars->mma_done, 0, status, KERR_WAIT_FULL);
+        }
+    } else if (warp < 6) {
+        // ------------------------------------------------------------ splitters
+        const int quarter = warp & 3;  // TMEM lanes this warp may access
+        const uint32_t t_lane = (uint32_t)(quarter * 32) << 16;
+        RingPos s, a;
+        bool ok = true;
+        for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
+            for (int st = 0; ok && st < g.n; ++st) {
+                const ColStage &cs = g.st[st];
+                const int nkb = (cs.K + kCBK - 1) / kCBK;
+                for (int i = 0; ok && i < cs.tiles * nkb; ++i) {
+                    // every round of every slot is waited for and released, also those
+                    // without input: a parity tells two rounds apart, not three
+                    if (!(ok = mbar_wait(&bars->full[s.i], s.ph, status, KERR_WAIT_FULL))) break;
+                    if (st == 0) {
+                        const int left = cs.K - (i % nkb) * kCBK;
+                        const float *x = reinterpret_cast<const float *>(smem + s.i * g.slot_bytes) +
+                                         quarter * 32 + lane;
+                        for (int k0 = 0; k0 < kCBK && k0 < left; k0 += kCGran) {
+                            float v[kCGran];
+                            uint32_t w[2 * kCGran];
+#pragma unroll
+                            for (int k = 0; k < kCGran; ++k) v[k] = x[(k0 + k) * kCBN];
+#pragma unroll
+                            for (int k = 0; k < kCGran; ++k) {
+                                const float h = f32_to_tf32_rne(v[k]);
+                                w[k] = __float_as_uint(h);
+                                w[kCGran + k] = __float_as_uint(f32_to_tf32_rne(v[k] - h));
+                            }
+                            if (!(ok = mbar_wait(&bars->aempty[a.i], a.ph ^ 1, status, KERR_WAIT_EMPTY))) break;
+                            tc_fence_after();
+                            tmem_st_32x32b_x32(tmem_base + g.gran0 + a.i * kCGranCols + t_lane, w);
+                            tmem_st_wait();
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&bars->afull[a.i]);
+                            a.next(g.gran);
+                        }
+                        if (!ok) break;
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->empty[s.i]);
+                    s.next(g.ring);
+                }
+            }
+            if (c_aborted(bars)) break;
+        }
+        if (!ok) c_set_abort(bars);
+    } else {
+        // ------------------------------------------------------------ epilogues
+        const int quarter = warp & 3;
+        const uint32_t t_lane = (uint32_t)(quarter * 32) << 16;
+        uint32_t chunks = 0, tiles = 0;
+        bool ok = true;
+        for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
+            const int col = blk * kCBN + quarter * 32 + lane;
+            for (int st = 0; ok && st < g.n; ++st) {
+                const ColStage &cs = g.st[st];
+                const int nkb = (cs.K + kCBK - 1) / kCBK;
+                const int kchunk = cs.kchunk > 0 ? cs.kchunk : nkb;
+                const int nchunk = (nkb + kchunk - 1) / kchunk;
+                const int groups = cs.rows / 16;
+                const uint32_t acc = tmem_base + cs.acc + t_lane;
+                for (int t = 0; ok && t < cs.tiles; ++t, ++tiles) {
+                    float sum[16 * NC];
+#pragma unroll
+                    for (int j = 0; j < 16 * NC; ++j) sum[j] = 0.f;
+                    auto add = [&](uint32_t from) {
+#pragma unroll
+                        for (int c = 0; c < NC; ++c)
+                            if (c < groups) {
+                                uint32_t v[16];
+                                tmem_ld_32x32b_x16(from + c * 16, v);
+                                tmem_ld_wait();
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    sum[c * 16 + j] = sum[c * 16 + j] + __uint_as_float(v[j]);
+                            }
+                    };
+                    for (int i = 0; i < nchunk; ++i, ++chunks) {
+                        const uint32_t b = chunks & 1u;
+                        if (!(ok = mbar_wait(&bars->dfull[b], (chunks >> 1) & 1u, status, KERR_WAIT_ACC_FULL)))
+                            break;
+                        tc_fence_after();
+                        add(acc + (b ? 2 * cs.rows : 0));
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars->dempty[b]);
+                    }
+                    if (!ok || !(ok = mbar_wait(&bars->cfull, tiles & 1u, status, KERR_WAIT_ACC_FULL))) break;
+                    tc_fence_after();
+                    add(acc + cs.rows);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->drained);
+                    if (st + 1 < g.n) {
+                        // this column of the next stage's A: hi, then lo (rows past M are the
+                        // zero products of zero-filled weights)
+                        const uint32_t x = tmem_base + t_lane;
+#pragma unroll
+                        for (int c = 0; c < NC; ++c)
+                            if (c < groups) {
+                                uint32_t h[16], l[16];
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) {
+                                    const float hf = f32_to_tf32_rne(sum[c * 16 + j]);
+                                    h[j] = __float_as_uint(hf);
+                                    l[j] = __float_as_uint(f32_to_tf32_rne(sum[c * 16 + j] - hf));
+                                }
+                                tmem_st_32x32b_x16(x + c * 16, h);
+                                tmem_st_32x32b_x16(x + cs.rows + c * 16, l);
+                            }
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars->xready);
+                    } else if (col < g.N) {
+                        // rows of C: a warp stores 32 consecutive columns at a time
+                        const int m0 = t * cs.rows;
+                        float *cp = g.C + (size_t)m0 * g.ldc + col;
+#pragma unroll
+                        for (int j = 0; j < 16 * NC; ++j)
+                            if (j < cs.rows && m0 + j < cs.M) cp[(size_t)j * g.ldc] = sum[j];
+                    }
+                }
+            }
+            if (c_aborted(bars)) break;
+        }
+        if (!ok) c_set_abort(bars);
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc(tmem_base, g.tmem_cols);
+    }
+}
+
+// ------------------------------------------------------------------ host side
+
+namespace {
+
+int pad16(long m) { return (int)((m + 15) / 16 * 16); }
+
+// Tiles, TMEM columns and rings of a chain on one of the two builds; false where it
+// does not fit.
+bool column_layout(int n, const long *M, const long *K, bool small, ColArgs &A)
+{
+    const int rows_max = small ? kCSmallRows : kCRows;
+    const int cols = small ? 256 : 512;
+    const int usable = cols - 2 * kCGranCols;  // at least two granules
+    int end = 0, widest = 0;
+    for (int i = 0; i < n; ++i) {
+        ColStage &cs = A.st[i];
+        cs.M = (int)M[i];
+        cs.K = (int)K[i];
+        cs.acc = i > 0 ? 2 * A.st[i - 1].rows : 0;
+        cs.tiles = 1;
+        if (i + 1 < n) {
+            if (M[i] > rows_max) return false;
+            cs.rows = pad16(M[i]);
+        } else {
+            const int most = std::min(rows_max, (usable - cs.acc) / 3 / 16 * 16);
+            // a first stage that is the last would stream B once per tile
+            if (most < 16 || (n == 1 && M[i] > most)) return false;
+            cs.tiles = (int)((M[i] + most - 1) / most);
+            cs.rows = pad16((M[i] + cs.tiles - 1) / cs.tiles);
+        }
+        end = std::max(end, cs.acc + 3 * cs.rows);
+        widest = std::max(widest, cs.rows);
+    }
+    if (end > usable) return false;
+    A.n = n;
+    A.tmem_cols = cols;
+    A.gran0 = end;
+    A.gran = std::min(kCMaxGran, (cols - end) / kCGranCols);
+    A.slot_bytes = kCXBytes + 2 * widest * 128;
+    A.ring = std::min(kCMaxRing, ((small ? kCHalfSmem : kCMaxSmem) - kCFixed) / A.slot_bytes);
+    A.smem = A.ring * A.slot_bytes + kCFixed;
+    A.small = small;
+    return A.ring >= 3;
+}
+
+bool column_layout(int n, const long *M, const long *K, ColArgs &A)
+{
+    return column_layout(n, M, K, true, A) || column_layout(n, M, K, false, A);
+}
+
+}  // namespace
+
+// Clocks of both ways (a model, per the rates measured on B200): here every SM runs
+// whole blocks, a block's stages one after the other (three MMAs per 8 k, about 3000
+// clocks of hand-over per stage), or its share of the memory that B and C cross; the
+// launch-per-stage path splits B through memory (12 bytes a value) and then spreads
+// 128 x 128 tiles of each stage over all SMs, a k-block in about 1400 clocks, a stage's
+// launch and drain about 6000. Deep or tall stages on few columns stay there.
+bool column_preferred(long N, int n, const long *M, const long *K, int num_sms)
+{
+    if (n < 1 || n > kPanelMaxStages || N < 1 || N > (1l << 30)) return false;
+    for (int i = 0; i < n; ++i)
+        if (M[i] < 1 || K[i] < 1 || M[i] > (1l << 30) || K[i] > (1l << 30)) return false;
+    static thread_local ColArgs A;
+    if (!column_layout(n, M, K, A)) return false;
+    const double blocks = (double)((N + kCBN - 1) / kCBN);
+    double block = 0.0, staged = 12.0 * K[0] * N / 3300.0;
+    for (int i = 0; i < n; ++i) {
+        const ColStage &cs = A.st[i];
+        block += cs.tiles * ((cs.K + 7) / 8 * 3.0 * std::max(48.0, cs.rows / 2.0) + 3000.0);
+        const double tiles = (double)((M[i] + 127) / 128) * blocks;
+        staged += 6000.0 + std::ceil(tiles / num_sms) * ((K[i] + 31) / 32) * 1400.0;
+    }
+    const double per_sm = A.small ? 2.0 : 1.0;
+    const double here = std::max(std::ceil(blocks / (num_sms * per_sm)) * block,
+                                 4.0 * (K[0] + M[n - 1]) * N / 3300.0);
+    return here < staged;
+}
+
+cudaError_t launch_column(const PanelChainArgs &a, int num_sms, int *status, cudaStream_t s)
+{
+    // launch parameters of the last few operand sets (tensor maps encoded once)
+    static std::mutex mu;
+    struct Built {
+        PanelChainArgs key;
+        ColArgs g;
+    };
+    static std::vector<std::unique_ptr<Built>> built;
+    static unsigned long long known = 0;
+    static thread_local ColArgs g;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (!(known >> (dev & 63) & 1)) {
+            cudaError_t e = cudaFuncSetAttribute(tc_column_kernel<kCSmallRows / 16, 2>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kCHalfSmem);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(tc_column_kernel<kCRows / 16, 1>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kCMaxSmem);
+            if (e != cudaSuccess) return e;
+            known |= 1ull << (dev & 63);
+        }
+        Built *hit = nullptr;
+        for (size_t i = 0; i < built.size(); ++i)
+            if (memcmp(&built[i]->key, &a, sizeof a) == 0 && built[i]->g.status == status) {
+                std::unique_ptr<Built> b = std::move(built[i]);
+                built.erase(built.begin() + i);
+                built.push_back(std::move(b));
+                hit = built.back().get();
+                break;
+            }
+        if (!hit) {
+            std::unique_ptr<Built> b(new Built);
+            memcpy(&b->key, &a, sizeof a);
+            memset(&b->g, 0, sizeof b->g);
+            ColArgs &A = b->g;
+            if (!column_layout(a.n, a.M, a.K, A)) return cudaErrorNotSupported;
+            if (!make_map(&A.tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.B, a.K[0], a.N, a.ldb, kCBN, kCBK,
+                          CU_TENSOR_MAP_SWIZZLE_NONE))
+                return cudaErrorNotSupported;
+            for (int i = 0; i < a.n; ++i) {
+                ColStage &cs = A.st[i];
+                cs.kchunk = a.kchunk[i];
+                if (!make_map(&cs.tm_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.w_hi[i], a.M[i], a.K[i],
+                              a.ldw[i], kCBK, cs.rows) ||
+                    !make_map(&cs.tm_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, a.w_lo[i], a.M[i], a.K[i],
+                              a.ldw[i], kCBK, cs.rows))
+                    return cudaErrorNotSupported;
+            }
+            A.C = a.C;
+            A.ldc = a.ldc;
+            A.N = (int)a.N;
+            A.nblocks = (int)((a.N + kCBN - 1) / kCBN);
+            A.status = status;
+            if (built.size() >= 8) built.erase(built.begin());
+            built.push_back(std::move(b));
+            hit = built.back().get();
+        }
+        g = hit->g;  // a copy: the entry may go once the lock is released
+    }
+    const int grid = std::min(g.nblocks, num_sms * (g.small ? 2 : 1));
+    if (g.small)
+        tc_column_kernel<kCSmallRows / 16, 2><<<grid, kCThreads, g.smem, s>>>(g);
+    else
+        tc_column_kernel<kCRows / 16, 1><<<grid, kCThreads, g.smem, s>>>(g);
+    return cudaGetLastError();
+}
+
+}  // namespace fg

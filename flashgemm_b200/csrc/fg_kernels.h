@@ -286,6 +286,15 @@ cudaError_t launch_panel(const PanelChain *chains_dev, const uint32_t *blocks_de
 cudaError_t launch_panel_one(const PanelChainArgs &a, int num_sms, int *status, cudaStream_t s,
                              unsigned long long *trace = nullptr);
 
+// ------------------------------------------------------------------ column chains
+//
+// FP32 (3xTF32) chains whose intermediates have at most 144 rows keep them in tensor
+// memory (fg_column.cu): one CTA per 128-column block, B read once as it is, any K_1,
+// any last width. Operands as for a panel-resident chain (16-byte-aligned rows).
+// Whether a chain fits and is expected to run faster so than one launch per stage.
+bool column_preferred(long N, int n, const long *M, const long *K, int num_sms);
+cudaError_t launch_column(const PanelChainArgs &a, int num_sms, int *status, cudaStream_t s);
+
 // Plain FP32 SGEMM on CUDA cores: C = A * B, one FMA per k in increasing k;
 // with kblock > 0 each block of kblock k is summed from zero and added to C.
 struct FfmaArgs {
@@ -304,10 +313,6 @@ cudaError_t launch_ffma_sgemm(const FfmaArgs &a, int num_sms, cudaStream_t s);
 // rounded up to 4); 0 where it does not.
 size_t ffma_sgemm_workspace(long M, long N, long K, int kblock, int num_sms);
 
-// FP32 -> (hi, lo) TF32 split of a rows x cols matrix (leading dims ld_in / ld_out).
-cudaError_t launch_split_tf32(const float *in, long ld_in, float *hi, float *lo, long ld_out,
-                              long rows, long cols, cudaStream_t s);
-
 // INT8 weight preparation: copies W (M x K, ld_in) into dst (ld_out >= K + 4,
 // a multiple of 16), shifting rows [tail_lo, tail_hi) left by one k-quad
 // (zero-filling the last quad) and keeping their first quad at [K, K + 4).
@@ -315,13 +320,20 @@ cudaError_t launch_prep_int8_weights(const int8_t *src, long ld_in, uint8_t *dst
                                      long M, long K, long tail_lo, long tail_hi,
                                      cudaStream_t s);
 
-// FP32 -> (hi, lo) TF32 splits of many matrices in one launch (jobs in device memory).
+// FP32 -> (hi, lo) TF32 splits of matrices (rows x cols, leading dimensions ld_in /
+// ld_out): up to kSplitBatch in one launch, or many with the jobs in device memory.
 struct SplitJob {
     const float *in;
     long ld_in;
     float *hi, *lo;
     long ld_out, rows, cols;
 };
+constexpr int kSplitBatch = 8;
+struct SplitBatch {
+    SplitJob job[kSplitBatch];
+    int n = 0;
+};
+cudaError_t launch_split_tf32(const SplitBatch &b, cudaStream_t s);
 cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long max_elems,
                                    cudaStream_t s);
 
