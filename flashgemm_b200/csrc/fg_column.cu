@@ -35,8 +35,8 @@
 // warps 6-9 run the epilogues (a warp of each group per TMEM lane quarter). Accumulators
 // are [d0 | c | d1]: two chunk sums around the correction. TMEM from the bottom: stage
 // 0's accumulators, or a later stage's A operand and then its accumulators (dead and
-// live parts never meet: every MMA of a stage has completed, and a lane has read its
-// sums, before that lane's operand is written); the granule ring above all of them, so
+// live parts never meet: every MMA of a stage has completed, and every warp of a lane
+// quarter has read its sums, before the quarter's operand is written); the granule ring above all of them, so
 // that the next block's input is split while this block's last stages run. Every wait
 // is bounded (fg_ptx.cuh); no CTA waits on another.
 #include <cuda.h>
@@ -46,6 +46,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "fg_tc_common.cuh"
@@ -57,15 +58,15 @@ namespace {
 constexpr int kCBN = 128;                     // columns per block (MMA M)
 constexpr int kCBK = 32;                      // k per k-block (a 128-byte weight row)
 constexpr int kCXBytes = kCBN * kCBK * 4;     // a k-block of B: 32 rows of 128 floats
-constexpr int kCGran = 16;                    // k per granule of the A ring
-constexpr int kCGranCols = 2 * kCGran;        // its TMEM columns: hi, then lo
-constexpr int kCThreads = 320;
 constexpr int kCMaxRing = 8, kCMaxGran = 8;
+// Warps: TMA producer, MMA issuer, 4 splitters, EW epilogue warps
+__host__ __device__ constexpr int c_threads(int ew) { return 32 * (6 + ew); }
 constexpr int kCFixed = 512 + 1024;           // barriers, alignment
 constexpr int kCMaxSmem = 232448;
 constexpr int kCHalfSmem = 113 * 1024;        // two CTAs per SM
 // Two builds: up to 48 rows per tile (half of TMEM and of shared memory, two CTAs per
-// SM, so that one CTA's chain of stages fills the other's waits) and up to 144
+// SM, so that one CTA's chain of stages fills the other's waits; 4 epilogue warps) and up
+// to 144 (8 epilogue warps, two per TMEM lane quarter)
 constexpr int kCSmallRows = 48, kCRows = 144;
 
 struct ColStage {
@@ -82,7 +83,7 @@ struct alignas(64) ColArgs {
     long ldc;
     int n, N, nblocks;
     int ring, slot_bytes;      // shared-memory ring: B's k-block, then hi and lo weight boxes
-    int gran, gran0;           // A ring: granules, first TMEM column
+    int gran, gran_k, gran0;   // A ring: granules, k per granule (16 or 32), first TMEM column
     int tmem_cols, smem, small;
     int *status;
 };
@@ -91,7 +92,7 @@ struct __align__(8) ColBars {
     uint64_t full[kCMaxRing];                      // shared-memory ring: TMA bytes
     uint64_t empty[kCMaxRing];                     // MMAs retired, and the 4 splitter warps are past it
     uint64_t afull[kCMaxGran], aempty[kCMaxGran];  // A ring (4 splitter warps / MMAs retired)
-    uint64_t dfull[2], dempty[2];                  // chunk sums (MMAs retired / 4 epilogue warps)
+    uint64_t dfull[2], dempty[2];                  // chunk sums (MMAs retired / epilogue warps)
     uint64_t cfull;                                // a tile's MMAs have all retired
     uint64_t drained;                              // the epilogue warps have read all of the tile
     uint64_t xready;                               // the next stage's A operand is in place
@@ -119,9 +120,9 @@ struct RingPos {
 
 }  // namespace
 
-// NC: 16-row groups of the widest tile; PER: CTAs per SM
-template <int NC, int PER>
-__global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_constant__ ColArgs g)
+// NG: 16-row groups of the widest tile per epilogue warp; EW: epilogue warps; PER: CTAs per SM
+template <int NG, int EW, int PER>
+__global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __grid_constant__ ColArgs g)
 {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -130,6 +131,18 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
     int *status = g.status;
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
+
+    // k-block kb of a stage's tile t into ring slot i: the weights' boxes, and B's for stage 0
+    auto load = [&](int st, int blk, int t, int kb, int i) {
+        const ColStage &cs = g.st[st];
+        const int w_bytes = cs.rows * 128;
+        uint8_t *p = smem + i * g.slot_bytes;
+        mbar_arrive_expect_tx(&bars->full[i], 2u * w_bytes + (st == 0 ? kCXBytes : 0));
+        if (st == 0) tma_load_2d(p, &g.tm_x, &bars->full[i], blk * kCBN, kb * kCBK);
+        tma_load_2d(p + kCXBytes, &cs.tm_hi, &bars->full[i], kb * kCBK, t * cs.rows);
+        tma_load_2d(p + kCXBytes + w_bytes, &cs.tm_lo, &bars->full[i], kb * kCBK, t * cs.rows);
+    };
+    const int first_loads = min(g.ring, (g.st[0].K + kCBK - 1) / kCBK);
 
     if (threadIdx.x == 0) {
         for (int r = 0; r < kCMaxRing; ++r) {
@@ -142,16 +155,18 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
         }
         for (int d = 0; d < 2; ++d) {
             mbar_init(&bars->dfull[d], 1);
-            mbar_init(&bars->dempty[d], 4);
+            mbar_init(&bars->dempty[d], EW);
         }
         mbar_init(&bars->cfull, 1);
-        mbar_init(&bars->drained, 4);
-        mbar_init(&bars->xready, 4);
+        mbar_init(&bars->drained, EW);
+        mbar_init(&bars->xready, EW);
         mbar_init(&bars->mma_done, 1);
         bars->abort = 0;
         fence_mbar_init();
-        tma_prefetch_desc(&g.tm_x);
-        for (int i = 0; i < g.n; ++i) {
+        // the ring's first round needs no wait, and nobody else: under way before the
+        // CTA meets, and before the later stages' tensor maps are fetched
+        for (int kb = 0; kb < first_loads; ++kb) load(0, blockIdx.x, 0, kb, kb);
+        for (int i = 1; i < g.n; ++i) {
             tma_prefetch_desc(&g.st[i].tm_hi);
             tma_prefetch_desc(&g.st[i].tm_lo);
         }
@@ -166,28 +181,24 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
             RingPos s;
-            uint32_t pending = 0, pending_ph = 0;
+            uint32_t pending = (1u << first_loads) - 1, pending_ph = 0;
+            int skip = first_loads;
             for (int blk = blockIdx.x; blk < g.nblocks; blk += gridDim.x) {
                 for (int st = 0; st < g.n; ++st) {
-                    const ColStage &cs = g.st[st];
-                    const int nkb = (cs.K + kCBK - 1) / kCBK;
-                    const int w_bytes = cs.rows * 128;
-                    const uint32_t tx = 2u * w_bytes + (st == 0 ? kCXBytes : 0);
-                    for (int t = 0; t < cs.tiles; ++t)
-                        for (int kb = 0; kb < nkb; ++kb) {
+                    const int nkb = (g.st[st].K + kCBK - 1) / kCBK;
+                    for (int t = 0; t < g.st[st].tiles; ++t)
+                        for (int kb = 0; kb < nkb; ++kb, s.next(g.ring)) {
+                            if (skip > 0) {  // loaded above
+                                --skip;
+                                continue;
+                            }
                             if (!mbar_wait(&bars->empty[s.i], s.ph ^ 1, status, KERR_WAIT_EMPTY)) {
                                 c_set_abort(bars);
                                 goto producer_done;
                             }
-                            uint8_t *p = smem + s.i * g.slot_bytes;
-                            mbar_arrive_expect_tx(&bars->full[s.i], tx);
-                            if (st == 0) tma_load_2d(p, &g.tm_x, &bars->full[s.i], blk * kCBN, kb * kCBK);
-                            tma_load_2d(p + kCXBytes, &cs.tm_hi, &bars->full[s.i], kb * kCBK, t * cs.rows);
-                            tma_load_2d(p + kCXBytes + w_bytes, &cs.tm_lo, &bars->full[s.i], kb * kCBK,
-                                        t * cs.rows);
+                            load(st, blk, t, kb, s.i);
                             pending |= 1u << s.i;
                             pending_ph = (pending_ph & ~(1u << s.i)) | (s.ph << s.i);
-                            s.next(g.ring);
                         }
                 }
                 if (c_aborted(bars)) break;
@@ -204,23 +215,26 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
             RingPos s, a;
             uint32_t chunks = 0;  // chunk sums started: buffer chunks & 1, round chunks >> 1
             uint32_t tiles = 0, xr = 0;
+            // an MMA takes 48 clocks up to 96 rows: the loops below leave the issuing thread
+            // little else than additions of constants (descriptors differ in their low word)
             const uint64_t w_desc0 = smem_desc(smem_u32(smem) + kCXBytes, 16, 1024, SMEM_SW128);
+            const uint32_t w_hi32 = (uint32_t)(w_desc0 >> 32);
+            const int gran_cols = 2 * g.gran_k;
             bool ok = true;
             for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
                 for (int st = 0; ok && st < g.n; ++st) {
                     const ColStage &cs = g.st[st];
-                    const int nkb = (cs.K + kCBK - 1) / kCBK;
+                    const int K = cs.K, rows = cs.rows, ntiles = cs.tiles;
+                    const int nkb = (K + kCBK - 1) / kCBK;
                     const int kchunk = cs.kchunk > 0 ? cs.kchunk : nkb;
-                    const uint32_t idesc = make_idesc(1, 2, 2, 0, 0, kCBN, cs.rows);
-                    const uint64_t lo_off = (uint64_t)((cs.rows * 128) >> 4);
-                    const uint32_t acc = tmem_base + cs.acc, c_tmem = acc + cs.rows;
-                    // a later stage's A: hi at column 0, lo after the previous stage's padded rows
-                    const uint32_t x_lo = st > 0 ? (uint32_t)g.st[st - 1].rows : 0u;
+                    const uint32_t idesc = make_idesc(1, 2, 2, 0, 0, kCBN, rows);
+                    const uint32_t lo_off = (uint32_t)(rows * 128) >> 4;
+                    const uint32_t acc = tmem_base + cs.acc, c_tmem = acc + rows;
                     if (st > 0) {
                         ok = mbar_wait(&bars->xready, xr & 1u, status, KERR_WAIT_FULL);
                         ++xr;
                     }
-                    for (int t = 0; ok && t < cs.tiles; ++t, ++tiles) {
+                    for (int t = 0; ok && t < ntiles; ++t, ++tiles) {
                         // the accumulators (and what overlies them) are free once the tile before is read
                         if (!(ok = mbar_wait(&bars->drained, (tiles & 1u) ^ 1u, status, KERR_WAIT_ACC_EMPTY)))
                             break;
@@ -232,35 +246,53 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
                                 if (!(ok = mbar_wait(&bars->dempty[b], ((chunks >> 1) & 1u) ^ 1u, status,
                                                      KERR_WAIT_ACC_EMPTY)))
                                     break;
-                                d_tmem = acc + (b ? 2 * cs.rows : 0);
+                                d_tmem = acc + (b ? 2 * rows : 0);
                                 more_d = 0;
                                 left = kchunk;
                             }
                             if (!(ok = mbar_wait(&bars->full[s.i], s.ph, status, KERR_WAIT_FULL))) break;
-                            tc_fence_after();
-                            const uint64_t w = w_desc0 + (uint64_t)((s.i * g.slot_bytes) >> 4);
-                            const int steps = min(4, (cs.K - kb * kCBK + 7) / 8);  // 8 k each
-                            auto step = [&](uint32_t hi, uint32_t lo, int k) {
-                                const uint64_t wk = w + (uint64_t)(k * 2);
-                                tc_mma_ts_tf32(c_tmem, lo, wk, idesc, more_c);
-                                tc_mma_ts_tf32(c_tmem, hi, wk + lo_off, idesc, 1);
-                                tc_mma_ts_tf32(d_tmem, hi, wk, idesc, more_d);
+                            const uint32_t w = (uint32_t)w_desc0 + ((uint32_t)(s.i * g.slot_bytes) >> 4);
+                            const uint32_t wl = w + lo_off;
+                            // step k of 8: A's columns at x (hi) and xl (lo), the weights' bytes 32 k on
+                            auto step = [&](uint32_t x, uint32_t xl, int k) {
+                                tc_mma_ts_tf32(c_tmem, xl, w + 2 * k, w_hi32, idesc, more_c);
+                                tc_mma_ts_tf32(c_tmem, x, wl + 2 * k, w_hi32, idesc, 1);
+                                tc_mma_ts_tf32(d_tmem, x, w + 2 * k, w_hi32, idesc, more_d);
                                 more_c = more_d = 1;
                             };
-                            if (st == 0) {
-                                for (int k0 = 0; k0 < steps; k0 += 2) {
+                            const int left_k = K - kb * kCBK;
+                            if (st == 0 && g.gran_k == 16) {
+                                for (int k0 = 0; k0 < 4 && k0 * 8 < left_k; k0 += 2) {
                                     if (!(ok = mbar_wait(&bars->afull[a.i], a.ph, status, KERR_WAIT_FULL))) break;
                                     tc_fence_after();
-                                    const uint32_t x = tmem_base + g.gran0 + a.i * kCGranCols;
-                                    step(x, x + kCGran, k0);
-                                    if (k0 + 1 < steps) step(x + 8, x + kCGran + 8, k0 + 1);
+                                    const uint32_t x = tmem_base + g.gran0 + a.i * 32;
+                                    step(x, x + 16, k0);
+                                    if (k0 * 8 + 8 < left_k) step(x + 8, x + 24, k0 + 1);
                                     tc_commit(&bars->aempty[a.i]);
                                     a.next(g.gran);
                                 }
                                 if (!ok) break;
                             } else {
-                                const uint32_t x = tmem_base + kb * kCBK;
-                                for (int k = 0; k < steps; ++k) step(x + 8 * k, x + x_lo + 8 * k, k);
+                                uint32_t x, xl;
+                                if (st == 0) {
+                                    if (!(ok = mbar_wait(&bars->afull[a.i], a.ph, status, KERR_WAIT_FULL))) break;
+                                    x = tmem_base + g.gran0 + a.i * gran_cols;
+                                    xl = x + kCBK;
+                                } else {  // hi at column 0, lo after the previous stage's padded rows
+                                    x = tmem_base + kb * kCBK;
+                                    xl = x + g.st[st - 1].rows;
+                                }
+                                tc_fence_after();
+                                if (left_k >= kCBK) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) step(x + 8 * k, xl + 8 * k, k);
+                                } else {
+                                    for (int k = 0; k * 8 < left_k; ++k) step(x + 8 * k, xl + 8 * k, k);
+                                }
+                                if (st == 0) {
+                                    tc_commit(&bars->aempty[a.i]);
+                                    a.next(g.gran);
+                                }
                             }
                             tc_commit(&bars->empty[s.i]);
                             s.next(g.ring);
@@ -285,38 +317,52 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
         const int quarter = warp & 3;  // TMEM lanes this warp may access
         const uint32_t t_lane = (uint32_t)(quarter * 32) << 16;
         RingPos s, a;
+        const int gran_cols = 2 * g.gran_k;
         bool ok = true;
+        // G k of this thread's column into the next granule: hi, then lo
+        auto put = [&](const float *x, auto g_tag) -> bool {
+            constexpr int G = decltype(g_tag)::value;
+            uint32_t h[G], l[G];
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                const float v = x[k * kCBN], hf = f32_to_tf32_rne(v);
+                h[k] = __float_as_uint(hf);
+                l[k] = __float_as_uint(f32_to_tf32_rne(v - hf));
+            }
+            if (!mbar_wait(&bars->aempty[a.i], a.ph ^ 1, status, KERR_WAIT_EMPTY)) return false;
+            tc_fence_after();
+            const uint32_t to = tmem_base + g.gran0 + a.i * gran_cols + t_lane;
+            if constexpr (G == 32) {
+                tmem_st_32x32b_x32(to, h);
+                tmem_st_32x32b_x32(to + 32, l);
+            } else {
+                tmem_st_32x32b_x16(to, h);
+                tmem_st_32x32b_x16(to + 16, l);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->afull[a.i]);
+            a.next(g.gran);
+            return true;
+        };
         for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
             for (int st = 0; ok && st < g.n; ++st) {
-                const ColStage &cs = g.st[st];
-                const int nkb = (cs.K + kCBK - 1) / kCBK;
-                for (int i = 0; ok && i < cs.tiles * nkb; ++i) {
+                const int K = g.st[st].K, nkb = (K + kCBK - 1) / kCBK;
+                const int rounds = g.st[st].tiles * nkb;
+                for (int i = 0; i < rounds; ++i) {
                     // every round of every slot is waited for and released, also those
                     // without input: a parity tells two rounds apart, not three
                     if (!(ok = mbar_wait(&bars->full[s.i], s.ph, status, KERR_WAIT_FULL))) break;
-                    if (st == 0) {
-                        const int left = cs.K - (i % nkb) * kCBK;
+                    if (st == 0) {  // one tile: i is the k-block (rows past K are zeros)
                         const float *x = reinterpret_cast<const float *>(smem + s.i * g.slot_bytes) +
                                          quarter * 32 + lane;
-                        for (int k0 = 0; k0 < kCBK && k0 < left; k0 += kCGran) {
-                            float v[kCGran];
-                            uint32_t w[2 * kCGran];
-#pragma unroll
-                            for (int k = 0; k < kCGran; ++k) v[k] = x[(k0 + k) * kCBN];
-#pragma unroll
-                            for (int k = 0; k < kCGran; ++k) {
-                                const float h = f32_to_tf32_rne(v[k]);
-                                w[k] = __float_as_uint(h);
-                                w[kCGran + k] = __float_as_uint(f32_to_tf32_rne(v[k] - h));
-                            }
-                            if (!(ok = mbar_wait(&bars->aempty[a.i], a.ph ^ 1, status, KERR_WAIT_EMPTY))) break;
-                            tc_fence_after();
-                            tmem_st_32x32b_x32(tmem_base + g.gran0 + a.i * kCGranCols + t_lane, w);
-                            tmem_st_wait();
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&bars->afull[a.i]);
-                            a.next(g.gran);
+                        if (g.gran_k == 32) {
+                            ok = put(x, std::integral_constant<int, 32>{});
+                        } else {
+                            ok = put(x, std::integral_constant<int, 16>{});
+                            if (ok && K - i * kCBK > 16)
+                                ok = put(x + 16 * kCBN, std::integral_constant<int, 16>{});
                         }
                         if (!ok) break;
                     }
@@ -331,6 +377,8 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
     } else {
         // ------------------------------------------------------------ epilogues
         const int quarter = warp & 3;
+        constexpr int STEP = EW / 4;              // warps that share a lane quarter
+        const int first = (warp - 6) >> 2;        // this warp's 16-row groups: first, first + STEP, ...
         const uint32_t t_lane = (uint32_t)(quarter * 32) << 16;
         uint32_t chunks = 0, tiles = 0;
         bool ok = true;
@@ -344,19 +392,19 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
                 const int groups = cs.rows / 16;
                 const uint32_t acc = tmem_base + cs.acc + t_lane;
                 for (int t = 0; ok && t < cs.tiles; ++t, ++tiles) {
-                    float sum[16 * NC];
+                    float sum[16 * NG];
 #pragma unroll
-                    for (int j = 0; j < 16 * NC; ++j) sum[j] = 0.f;
+                    for (int j = 0; j < 16 * NG; ++j) sum[j] = 0.f;
                     auto add = [&](uint32_t from) {
 #pragma unroll
-                        for (int c = 0; c < NC; ++c)
-                            if (c < groups) {
+                        for (int i = 0; i < NG; ++i)
+                            if (first + i * STEP < groups) {
                                 uint32_t v[16];
-                                tmem_ld_32x32b_x16(from + c * 16, v);
+                                tmem_ld_32x32b_x16(from + (first + i * STEP) * 16, v);
                                 tmem_ld_wait();
 #pragma unroll
                                 for (int j = 0; j < 16; ++j)
-                                    sum[c * 16 + j] = sum[c * 16 + j] + __uint_as_float(v[j]);
+                                    sum[i * 16 + j] = sum[i * 16 + j] + __uint_as_float(v[j]);
                             }
                     };
                     for (int i = 0; i < nchunk; ++i, ++chunks) {
@@ -377,20 +425,25 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
                     if (lane == 0) mbar_arrive(&bars->drained);
                     if (st + 1 < g.n) {
                         // this column of the next stage's A: hi, then lo (rows past M are the
-                        // zero products of zero-filled weights)
+                        // zero products of zero-filled weights). It may overlie sums that the
+                        // other warp of these lanes still reads.
+                        if (STEP > 1 &&
+                            !(ok = mbar_wait(&bars->drained, tiles & 1u, status, KERR_WAIT_ACC_FULL)))
+                            break;
                         const uint32_t x = tmem_base + t_lane;
 #pragma unroll
-                        for (int c = 0; c < NC; ++c)
-                            if (c < groups) {
+                        for (int i = 0; i < NG; ++i)
+                            if (first + i * STEP < groups) {
                                 uint32_t h[16], l[16];
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) {
-                                    const float hf = f32_to_tf32_rne(sum[c * 16 + j]);
+                                    const float hf = f32_to_tf32_rne(sum[i * 16 + j]);
                                     h[j] = __float_as_uint(hf);
-                                    l[j] = __float_as_uint(f32_to_tf32_rne(sum[c * 16 + j] - hf));
+                                    l[j] = __float_as_uint(f32_to_tf32_rne(sum[i * 16 + j] - hf));
                                 }
-                                tmem_st_32x32b_x16(x + c * 16, h);
-                                tmem_st_32x32b_x16(x + cs.rows + c * 16, l);
+                                const uint32_t at = x + (first + i * STEP) * 16;
+                                tmem_st_32x32b_x16(at, h);
+                                tmem_st_32x32b_x16(at + cs.rows, l);
                             }
                         tmem_st_wait();
                         tc_fence_before();
@@ -398,11 +451,15 @@ __global__ void __launch_bounds__(kCThreads, PER) tc_column_kernel(const __grid_
                         if (lane == 0) mbar_arrive(&bars->xready);
                     } else if (col < g.N) {
                         // rows of C: a warp stores 32 consecutive columns at a time
-                        const int m0 = t * cs.rows;
-                        float *cp = g.C + (size_t)m0 * g.ldc + col;
 #pragma unroll
-                        for (int j = 0; j < 16 * NC; ++j)
-                            if (j < cs.rows && m0 + j < cs.M) cp[(size_t)j * g.ldc] = sum[j];
+                        for (int i = 0; i < NG; ++i) {
+                            const int r0 = (first + i * STEP) * 16;  // row in the tile
+                            const int m = min(cs.rows, cs.M - t * cs.rows) - r0;
+                            float *cp = g.C + (size_t)(t * cs.rows + r0) * g.ldc + col;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j)
+                                if (j < m) cp[(size_t)j * g.ldc] = sum[i * 16 + j];
+                        }
                     }
                 }
             }
@@ -432,7 +489,7 @@ bool column_layout(int n, const long *M, const long *K, bool small, ColArgs &A)
 {
     const int rows_max = small ? kCSmallRows : kCRows;
     const int cols = small ? 256 : 512;
-    const int usable = cols - 2 * kCGranCols;  // at least two granules
+    const int usable = cols - 2 * 32;  // at least two granules of 16 k
     int end = 0, widest = 0;
     for (int i = 0; i < n; ++i) {
         ColStage &cs = A.st[i];
@@ -457,7 +514,8 @@ bool column_layout(int n, const long *M, const long *K, bool small, ColArgs &A)
     A.n = n;
     A.tmem_cols = cols;
     A.gran0 = end;
-    A.gran = std::min(kCMaxGran, (cols - end) / kCGranCols);
+    A.gran_k = cols - end >= 2 * 64 ? 32 : 16;  // whole k-blocks where two of them fit
+    A.gran = std::min(kCMaxGran, (cols - end) / (2 * A.gran_k));
     A.slot_bytes = kCXBytes + 2 * widest * 128;
     A.ring = std::min(kCMaxRing, ((small ? kCHalfSmem : kCMaxSmem) - kCFixed) / A.slot_bytes);
     A.smem = A.ring * A.slot_bytes + kCFixed;
@@ -515,10 +573,10 @@ cudaError_t launch_column(const PanelChainArgs &a, int num_sms, int *status, cud
         int dev = 0;
         cudaGetDevice(&dev);
         if (!(known >> (dev & 63) & 1)) {
-            cudaError_t e = cudaFuncSetAttribute(tc_column_kernel<kCSmallRows / 16, 2>,
+            cudaError_t e = cudaFuncSetAttribute(tc_column_kernel<kCSmallRows / 16, 4, 2>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, kCHalfSmem);
             if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(tc_column_kernel<kCRows / 16, 1>,
+                e = cudaFuncSetAttribute(tc_column_kernel<(kCRows / 16 + 1) / 2, 8, 1>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kCMaxSmem);
             if (e != cudaSuccess) return e;
             known |= 1ull << (dev & 63);
@@ -563,9 +621,9 @@ cudaError_t launch_column(const PanelChainArgs &a, int num_sms, int *status, cud
     }
     const int grid = std::min(g.nblocks, num_sms * (g.small ? 2 : 1));
     if (g.small)
-        tc_column_kernel<kCSmallRows / 16, 2><<<grid, kCThreads, g.smem, s>>>(g);
+        tc_column_kernel<kCSmallRows / 16, 4, 2><<<grid, c_threads(4), g.smem, s>>>(g);
     else
-        tc_column_kernel<kCRows / 16, 1><<<grid, kCThreads, g.smem, s>>>(g);
+        tc_column_kernel<(kCRows / 16 + 1) / 2, 8, 1><<<grid, c_threads(8), g.smem, s>>>(g);
     return cudaGetLastError();
 }
 

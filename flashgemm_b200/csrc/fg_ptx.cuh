@@ -321,14 +321,15 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
 // B columns [0, N/2) come from this CTA's shared memory, A rows 128-255 and B
 // columns [N/2, N) from the peer's at the same offsets; D rows 0-127 land in
 // this CTA's TMEM, rows 128-255 in the peer's, at the same TMEM address.
-// TF32 with the A operand in TMEM: 128 lanes (rows of A), 8 columns (k) at a_tmem.
-__device__ __forceinline__ void tc_mma_ts_tf32(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                               uint32_t idesc, uint32_t accumulate)
+// TF32 with the A operand in TMEM: 128 lanes (rows of A), 8 columns (k) at a_tmem; the
+// descriptor of B by its two words.
+__device__ __forceinline__ void tc_mma_ts_tf32(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo,
+                                               uint32_t b_desc_hi, uint32_t idesc, uint32_t accumulate)
 {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate));
+        "{\n\t.reg .pred p;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], b, %4, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate));
 }
 
 template <MmaKind K>
