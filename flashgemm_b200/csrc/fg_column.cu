@@ -20,14 +20,17 @@
 // warps read it (a thread its own column, conflict-free) and put (hi, lo) into a ring
 // of 16-deep granules in TMEM. Only the weights are shared-memory operands.
 //
-// What bounds it: the tensor pipe (three TF32 MMAs per 8 k, 48 clocks each up to 96
-// rows, rows / 2 above) and, on many columns, reading B once. The launch-per-stage
+// What bounds it: the thread that issues the MMAs (about 70 clocks for each, 67 for a
+// commit, 96 for a wait that is already over) and the tensor pipe (three TF32 products
+// per 8 k of 48 clocks each up to 96 rows, rows / 2 above), hence one MMA for two of the
+// products where it fits, one commit per k-block, and waits tested ahead; and, on many columns, reading B once. The launch-per-stage
 // path that it replaces wrote B's split to memory and read it back (3x its bytes)
 // and paid a launch and a memory round trip per stage. Measured (B200, us a call, that
 // path -> this): SPLICE_NUMBERS
 //
 // The arithmetic is that path's: per 8 k the correction terms lo * hi, then hi * lo,
-// into their own accumulator and hi * hi into the chunk's; every `kchunk` k-blocks
+// into their own accumulator and hi * hi into the chunk's (hi * [hi | lo] as one MMA over the
+// stacked weights, into adjacent accumulators); every `kchunk` k-blocks
 // of 32 the chunk's sum goes to FP32 registers, the correction is added once at the
 // end; so the results are the same bits.
 //
@@ -74,6 +77,7 @@ struct ColStage {
     int M, K, kchunk;
     int rows, tiles;           // rows per tile (a multiple of 16); more than one tile: last stage only
     int acc;                   // TMEM column of its accumulators
+    int stack;                 // rows <= 128: hi and lo weights as one operand of 2 x rows
 };
 
 struct alignas(64) ColArgs {
@@ -84,6 +88,7 @@ struct alignas(64) ColArgs {
     int n, N, nblocks;
     int ring, slot_bytes;      // shared-memory ring: B's k-block, then hi and lo weight boxes
     int gran, gran_k, gran0;   // A ring: granules, k per granule (16 or 32), first TMEM column
+    int later_rounds;          // ring rounds of a block after its first stage
     int tmem_cols, smem, small;
     int *status;
 };
@@ -91,7 +96,7 @@ struct alignas(64) ColArgs {
 struct __align__(8) ColBars {
     uint64_t full[kCMaxRing];                      // shared-memory ring: TMA bytes
     uint64_t empty[kCMaxRing];                     // MMAs retired, and the 4 splitter warps are past it
-    uint64_t afull[kCMaxGran], aempty[kCMaxGran];  // A ring (4 splitter warps / MMAs retired)
+    uint64_t afull[kCMaxGran], aempty[kCMaxGran];  // A ring: 4 splitter warps / 16-deep granules: MMAs retired
     uint64_t dfull[2], dempty[2];                  // chunk sums (MMAs retired / epilogue warps)
     uint64_t cfull;                                // a tile's MMAs have all retired
     uint64_t drained;                              // the epilogue warps have read all of the tile
@@ -132,15 +137,21 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    // k-block kb of a stage's tile t into ring slot i: the weights' boxes, and B's for stage 0
-    auto load = [&](int st, int blk, int t, int kb, int i) {
+    // k-block kb of a stage's tile t into ring slot i: the weights' boxes, and B's for stage 0.
+    // Weights lie (hi, lo) for a chunk summed in [d0 | c], (lo, hi) for one in [c | d1].
+    auto load = [&](int st, int blk, int t, int kb, int i, bool lo_first) {
         const ColStage &cs = g.st[st];
         const int w_bytes = cs.rows * 128;
         uint8_t *p = smem + i * g.slot_bytes;
         mbar_arrive_expect_tx(&bars->full[i], 2u * w_bytes + (st == 0 ? kCXBytes : 0));
         if (st == 0) tma_load_2d(p, &g.tm_x, &bars->full[i], blk * kCBN, kb * kCBK);
-        tma_load_2d(p + kCXBytes, &cs.tm_hi, &bars->full[i], kb * kCBK, t * cs.rows);
-        tma_load_2d(p + kCXBytes + w_bytes, &cs.tm_lo, &bars->full[i], kb * kCBK, t * cs.rows);
+        tma_load_2d(p + kCXBytes, lo_first ? &cs.tm_lo : &cs.tm_hi, &bars->full[i], kb * kCBK, t * cs.rows);
+        tma_load_2d(p + kCXBytes + w_bytes, lo_first ? &cs.tm_hi : &cs.tm_lo, &bars->full[i], kb * kCBK,
+                    t * cs.rows);
+    };
+    auto chunk_blocks = [&](int st) {
+        const int nkb = (g.st[st].K + kCBK - 1) / kCBK;
+        return g.st[st].kchunk > 0 ? g.st[st].kchunk : nkb;
     };
     const int first_loads = min(g.ring, (g.st[0].K + kCBK - 1) / kCBK);
 
@@ -165,7 +176,8 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
         fence_mbar_init();
         // the ring's first round needs no wait, and nobody else: under way before the
         // CTA meets, and before the later stages' tensor maps are fetched
-        for (int kb = 0; kb < first_loads; ++kb) load(0, blockIdx.x, 0, kb, kb);
+        for (int kb = 0; kb < first_loads; ++kb)
+            load(0, blockIdx.x, 0, kb, kb, (kb / chunk_blocks(0)) & 1);
         for (int i = 1; i < g.n; ++i) {
             tma_prefetch_desc(&g.st[i].tm_hi);
             tma_prefetch_desc(&g.st[i].tm_lo);
@@ -183,10 +195,11 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
             RingPos s;
             uint32_t pending = (1u << first_loads) - 1, pending_ph = 0;
             int skip = first_loads;
+            uint32_t chunks = 0;  // chunks of the tiles before
             for (int blk = blockIdx.x; blk < g.nblocks; blk += gridDim.x) {
                 for (int st = 0; st < g.n; ++st) {
-                    const int nkb = (g.st[st].K + kCBK - 1) / kCBK;
-                    for (int t = 0; t < g.st[st].tiles; ++t)
+                    const int nkb = (g.st[st].K + kCBK - 1) / kCBK, kchunk = chunk_blocks(st);
+                    for (int t = 0; t < g.st[st].tiles; ++t, chunks += (nkb + kchunk - 1) / kchunk)
                         for (int kb = 0; kb < nkb; ++kb, s.next(g.ring)) {
                             if (skip > 0) {  // loaded above
                                 --skip;
@@ -196,7 +209,7 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
                                 c_set_abort(bars);
                                 goto producer_done;
                             }
-                            load(st, blk, t, kb, s.i);
+                            load(st, blk, t, kb, s.i, (chunks + kb / kchunk) & 1u);
                             pending |= 1u << s.i;
                             pending_ph = (pending_ph & ~(1u << s.i)) | (s.ph << s.i);
                         }
@@ -215,84 +228,113 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
             RingPos s, a;
             uint32_t chunks = 0;  // chunk sums started: buffer chunks & 1, round chunks >> 1
             uint32_t tiles = 0, xr = 0;
-            // an MMA takes 48 clocks up to 96 rows: the loops below leave the issuing thread
-            // little else than additions of constants (descriptors differ in their low word)
             const uint64_t w_desc0 = smem_desc(smem_u32(smem) + kCXBytes, 16, 1024, SMEM_SW128);
-            const uint32_t w_hi32 = (uint32_t)(w_desc0 >> 32);
-            const int gran_cols = 2 * g.gran_k;
+            const uint32_t w_hi32 = (uint32_t)(w_desc0 >> 32);  // descriptors differ in the low word
+            const bool whole = g.gran_k == 32;  // a granule is a k-block
             bool ok = true;
             for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
                 for (int st = 0; ok && st < g.n; ++st) {
                     const ColStage &cs = g.st[st];
                     const int K = cs.K, rows = cs.rows, ntiles = cs.tiles;
                     const int nkb = (K + kCBK - 1) / kCBK;
-                    const int kchunk = cs.kchunk > 0 ? cs.kchunk : nkb;
+                    const int kchunk = chunk_blocks(st);
+                    const bool stack = cs.stack, first = st == 0;
                     const uint32_t idesc = make_idesc(1, 2, 2, 0, 0, kCBN, rows);
-                    const uint32_t lo_off = (uint32_t)(rows * 128) >> 4;
+                    const uint32_t idesc2 = make_idesc(1, 2, 2, 0, 0, kCBN, stack ? 2 * rows : rows);
+                    const uint32_t half = (uint32_t)(rows * 128) >> 4;
                     const uint32_t acc = tmem_base + cs.acc, c_tmem = acc + rows;
-                    if (st > 0) {
+                    const uint32_t x_rows = first ? 0u : (uint32_t)g.st[st - 1].rows;
+                    if (!first) {
                         ok = mbar_wait(&bars->xready, xr & 1u, status, KERR_WAIT_FULL);
                         ++xr;
                     }
+                    // the barrier that says a k-block's operands are in place: its granule (the
+                    // splitters waited for the slot's bytes, weights included) or its slot
+                    auto ready_bar = [&](bool next) -> uint64_t * {
+                        const RingPos &r = first ? a : s;
+                        const int n = first ? g.gran : g.ring;
+                        const int i = !next ? r.i : r.i + 1 == n ? 0 : r.i + 1;
+                        return first ? &bars->afull[i] : &bars->full[i];
+                    };
+                    auto ready_ph = [&](bool next) -> uint32_t {
+                        const RingPos &r = first ? a : s;
+                        const int n = first ? g.gran : g.ring;
+                        return next && r.i + 1 == n ? r.ph ^ 1 : r.ph;
+                    };
                     for (int t = 0; ok && t < ntiles; ++t, ++tiles) {
                         // the accumulators (and what overlies them) are free once the tile before is read
                         if (!(ok = mbar_wait(&bars->drained, (tiles & 1u) ^ 1u, status, KERR_WAIT_ACC_EMPTY)))
                             break;
-                        uint32_t more_c = 0, more_d = 0, d_tmem = acc;
+                        uint32_t more_c = 0, d_tmem = acc, s_tmem = acc, hi_off = 0, lo_off = half;
                         int left = 0;  // k-blocks left of the chunk
+                        bool ready = false, free_d = false;  // waits found to be over ahead of time
                         for (int kb = 0; kb < nkb; ++kb) {
-                            if (left == 0) {
+                            const bool begin = left == 0;
+                            if (begin) {
                                 const uint32_t b = chunks & 1u;
-                                if (!(ok = mbar_wait(&bars->dempty[b], ((chunks >> 1) & 1u) ^ 1u, status,
-                                                     KERR_WAIT_ACC_EMPTY)))
+                                if (!free_d && !(ok = mbar_wait(&bars->dempty[b], ((chunks >> 1) & 1u) ^ 1u,
+                                                                status, KERR_WAIT_ACC_EMPTY)))
                                     break;
+                                free_d = false;
                                 d_tmem = acc + (b ? 2 * rows : 0);
-                                more_d = 0;
+                                s_tmem = b ? c_tmem : acc;  // [c | d1] or [d0 | c]
+                                hi_off = b ? half : 0;
+                                lo_off = b ? 0 : half;
                                 left = kchunk;
                             }
-                            if (!(ok = mbar_wait(&bars->full[s.i], s.ph, status, KERR_WAIT_FULL))) break;
-                            const uint32_t w = (uint32_t)w_desc0 + ((uint32_t)(s.i * g.slot_bytes) >> 4);
-                            const uint32_t wl = w + lo_off;
-                            // step k of 8: A's columns at x (hi) and xl (lo), the weights' bytes 32 k on
-                            auto step = [&](uint32_t x, uint32_t xl, int k) {
-                                tc_mma_ts_tf32(c_tmem, xl, w + 2 * k, w_hi32, idesc, more_c);
-                                tc_mma_ts_tf32(c_tmem, x, wl + 2 * k, w_hi32, idesc, 1);
-                                tc_mma_ts_tf32(d_tmem, x, w + 2 * k, w_hi32, idesc, more_d);
-                                more_c = more_d = 1;
-                            };
+                            const uint32_t w0 = (uint32_t)w_desc0 + ((uint32_t)(s.i * g.slot_bytes) >> 4);
+                            const uint32_t wh = w0 + hi_off, wl = w0 + lo_off;
                             const int left_k = K - kb * kCBK;
-                            if (st == 0 && g.gran_k == 16) {
+                            // step k of 8: A's columns at x (hi) and xl (lo), the weights' bytes 32 k on
+                            auto step3 = [&](uint32_t x, uint32_t xl, int k, uint32_t more_d) {
+                                tc_mma_ts_tf32(c_tmem, xl, wh + 2 * k, w_hi32, idesc, more_c);
+                                tc_mma_ts_tf32(c_tmem, x, wl + 2 * k, w_hi32, idesc, 1);
+                                tc_mma_ts_tf32(d_tmem, x, wh + 2 * k, w_hi32, idesc, more_d);
+                                more_c = 1;
+                            };
+                            if (first && !whole) {
                                 for (int k0 = 0; k0 < 4 && k0 * 8 < left_k; k0 += 2) {
-                                    if (!(ok = mbar_wait(&bars->afull[a.i], a.ph, status, KERR_WAIT_FULL))) break;
+                                    if (!ready &&
+                                        !(ok = mbar_wait(&bars->afull[a.i], a.ph, status, KERR_WAIT_FULL)))
+                                        break;
                                     tc_fence_after();
+                                    ready = mbar_test(ready_bar(true), ready_ph(true));
                                     const uint32_t x = tmem_base + g.gran0 + a.i * 32;
-                                    step(x, x + 16, k0);
-                                    if (k0 * 8 + 8 < left_k) step(x + 8, x + 24, k0 + 1);
+                                    step3(x, x + 16, k0, !begin || k0);
+                                    if (k0 * 8 + 8 < left_k) step3(x + 8, x + 24, k0 + 1, 1);
                                     tc_commit(&bars->aempty[a.i]);
                                     a.next(g.gran);
                                 }
                                 if (!ok) break;
                             } else {
-                                uint32_t x, xl;
-                                if (st == 0) {
-                                    if (!(ok = mbar_wait(&bars->afull[a.i], a.ph, status, KERR_WAIT_FULL))) break;
-                                    x = tmem_base + g.gran0 + a.i * gran_cols;
-                                    xl = x + kCBK;
-                                } else {  // hi at column 0, lo after the previous stage's padded rows
-                                    x = tmem_base + kb * kCBK;
-                                    xl = x + g.st[st - 1].rows;
-                                }
+                                if (!ready && !(ok = mbar_wait(ready_bar(false), ready_ph(false), status,
+                                                               KERR_WAIT_FULL)))
+                                    break;
                                 tc_fence_after();
-                                if (left_k >= kCBK) {
+                                // asked now, looked at after this k-block's MMAs are issued
+                                ready = mbar_test(ready_bar(true), ready_ph(true));
+                                // hi at column 0 and lo after the previous stage's padded rows, or a granule
+                                const uint32_t x = tmem_base + (first ? g.gran0 + a.i * 64 : kb * kCBK);
+                                const uint32_t xl = x + (first ? (uint32_t)kCBK : x_rows);
+                                auto step2 = [&](int k) {
+                                    tc_mma_ts_tf32(c_tmem, xl + 8 * k, wh + 2 * k, w_hi32, idesc, 1);
+                                    tc_mma_ts_tf32(s_tmem, x + 8 * k, w0 + 2 * k, w_hi32, idesc2, 1);
+                                };
+                                // a chunk's first step starts its sum, while the correction runs on
+                                if (begin || !stack)
+                                    step3(x, xl, 0, !begin);
+                                else
+                                    step2(0);
+                                if (stack && left_k >= kCBK) {
 #pragma unroll
-                                    for (int k = 0; k < 4; ++k) step(x + 8 * k, xl + 8 * k, k);
+                                    for (int k = 1; k < 4; ++k) step2(k);
+                                } else if (left_k >= kCBK) {
+#pragma unroll
+                                    for (int k = 1; k < 4; ++k) step3(x + 8 * k, xl + 8 * k, k, 1);
                                 } else {
-                                    for (int k = 0; k * 8 < left_k; ++k) step(x + 8 * k, xl + 8 * k, k);
+                                    for (int k = 1; k * 8 < left_k; ++k) step3(x + 8 * k, xl + 8 * k, k, 1);
                                 }
-                                if (st == 0) {
-                                    tc_commit(&bars->aempty[a.i]);
-                                    a.next(g.gran);
-                                }
+                                if (first) a.next(g.gran);
                             }
                             tc_commit(&bars->empty[s.i]);
                             s.next(g.ring);
@@ -300,6 +342,7 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
                                 tc_commit(&bars->dfull[chunks & 1u]);
                                 ++chunks;
                                 left = 0;
+                                if (kb + 1 < nkb) free_d = mbar_test(&bars->dempty[chunks & 1u], ((chunks >> 1) & 1u) ^ 1u);
                             }
                         }
                         if (!ok) break;
@@ -319,8 +362,9 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
         RingPos s, a;
         const int gran_cols = 2 * g.gran_k;
         bool ok = true;
-        // G k of this thread's column into the next granule: hi, then lo
-        auto put = [&](const float *x, auto g_tag) -> bool {
+        // G k of this thread's column into the next granule: hi, then lo, once the MMAs
+        // that read it last have retired (free: that is known)
+        auto put = [&](const float *x, auto g_tag, uint64_t *used, uint32_t used_ph, bool free) -> bool {
             constexpr int G = decltype(g_tag)::value;
             uint32_t h[G], l[G];
 #pragma unroll
@@ -329,7 +373,7 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
                 h[k] = __float_as_uint(hf);
                 l[k] = __float_as_uint(f32_to_tf32_rne(v - hf));
             }
-            if (!mbar_wait(&bars->aempty[a.i], a.ph ^ 1, status, KERR_WAIT_EMPTY)) return false;
+            if (!free && !mbar_wait(used, used_ph, status, KERR_WAIT_EMPTY)) return false;
             tc_fence_after();
             const uint32_t to = tmem_base + g.gran0 + a.i * gran_cols + t_lane;
             if constexpr (G == 32) {
@@ -346,6 +390,10 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
             a.next(g.gran);
             return true;
         };
+        // The k-block that used a whole granule before: g.gran rounds ago in this block's first
+        // stage, else in the last block's, its later rounds in between. Its slot's empty
+        // barrier says when its MMAs have retired; further back than the ring is long,
+        // the slot has been filled anew and waited for since.
         for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
             for (int st = 0; ok && st < g.n; ++st) {
                 const int K = g.st[st].K, nkb = (K + kCBK - 1) / kCBK;
@@ -358,11 +406,21 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
                         const float *x = reinterpret_cast<const float *>(smem + s.i * g.slot_bytes) +
                                          quarter * 32 + lane;
                         if (g.gran_k == 32) {
-                            ok = put(x, std::integral_constant<int, 32>{});
+                            const int back = g.gran + (i < g.gran ? g.later_rounds : 0);
+                            const bool free = (blk == (int)blockIdx.x && i < g.gran) || back > g.ring;
+                            // round s - back: the ring is at least as long, so at most one turn ago
+                            int j = s.i - back;
+                            uint32_t ph = s.ph;
+                            if (j < 0) {
+                                j += g.ring;
+                                ph ^= 1;
+                            }
+                            ok = put(x, std::integral_constant<int, 32>{}, &bars->empty[free ? 0 : j], ph, free);
                         } else {
-                            ok = put(x, std::integral_constant<int, 16>{});
+                            ok = put(x, std::integral_constant<int, 16>{}, &bars->aempty[a.i], a.ph ^ 1, false);
                             if (ok && K - i * kCBK > 16)
-                                ok = put(x + 16 * kCBN, std::integral_constant<int, 16>{});
+                                ok = put(x + 16 * kCBN, std::integral_constant<int, 16>{}, &bars->aempty[a.i],
+                                         a.ph ^ 1, false);
                         }
                         if (!ok) break;
                     }
@@ -490,7 +548,7 @@ bool column_layout(int n, const long *M, const long *K, bool small, ColArgs &A)
     const int rows_max = small ? kCSmallRows : kCRows;
     const int cols = small ? 256 : 512;
     const int usable = cols - 2 * 32;  // at least two granules of 16 k
-    int end = 0, widest = 0;
+    int end = 0, widest = 0, later = 0;
     for (int i = 0; i < n; ++i) {
         ColStage &cs = A.st[i];
         cs.M = (int)M[i];
@@ -507,7 +565,9 @@ bool column_layout(int n, const long *M, const long *K, bool small, ColArgs &A)
             cs.tiles = (int)((M[i] + most - 1) / most);
             cs.rows = pad16((M[i] + cs.tiles - 1) / cs.tiles);
         }
+        cs.stack = cs.rows <= 128;
         end = std::max(end, cs.acc + 3 * cs.rows);
+        if (i > 0) later += cs.tiles * ((cs.K + kCBK - 1) / kCBK);
         widest = std::max(widest, cs.rows);
     }
     if (end > usable) return false;
@@ -520,6 +580,9 @@ bool column_layout(int n, const long *M, const long *K, bool small, ColArgs &A)
     A.ring = std::min(kCMaxRing, ((small ? kCHalfSmem : kCMaxSmem) - kCFixed) / A.slot_bytes);
     A.smem = A.ring * A.slot_bytes + kCFixed;
     A.small = small;
+    A.later_rounds = later;
+    // a granule's last use is looked up at most one turn of the ring back
+    if (A.gran_k == 32) A.gran = std::min(A.gran, A.ring);
     return A.ring >= 3;
 }
 
