@@ -801,19 +801,19 @@ static cudaError_t launch_chain_op(const StageArgs *stages, int n, int *done, in
         c.opts = base;
         set_counters(st, 0u);
         list_schedule(sched_stages(st, G::BK).data(), n, pairs, 2.0, c.off, ent, &span_block,
-                      nullptr, &base);
+                      &base);
         c.stream = 0u;
         const unsigned mode = stream_mode();
         if (n > 1 && mode != 0u) {
             const unsigned mask = mode == kStreamAuto ? 0xffu : mode;
             set_counters(st, mask);
             const std::vector<SchedStage> ss = sched_stages(st, G::BK);
-            list_schedule(ss.data(), n, pairs, 2.0, off_s, ent_s, &span_stream, nullptr, &base);
+            list_schedule(ss.data(), n, pairs, 2.0, off_s, ent_s, &span_stream, &base);
             // feeders at a streamed boundary (see SchedOpts): the best of a small grid
             SchedOpts chosen = base;
             SchedOpts forced = base;
             if (feed_forced(forced) && forced.feed_stage + 1 < n && ((mask >> forced.feed_stage) & 1u)) {
-                list_schedule(ss.data(), n, pairs, 2.0, off_s, ent_s, &span_stream, nullptr, &forced);
+                list_schedule(ss.data(), n, pairs, 2.0, off_s, ent_s, &span_stream, &forced);
                 chosen = forced;
             } else if (feed_mode()) {
                 SchedOpts best = base;
@@ -829,12 +829,12 @@ static cudaError_t launch_chain_op(const StageArgs *stages, int n, int *done, in
                             fd.feed_workers = q;
                             fd.feed_rows = d;
                             double span_f = 0.0;
-                            list_schedule(ss.data(), n, pairs, 2.0, off_f, ent_f, &span_f, nullptr, &fd);
+                            list_schedule(ss.data(), n, pairs, 2.0, off_f, ent_f, &span_f, &fd);
                             if (span_f < span_best - 1e-9) span_best = span_f, best = fd;
                         }
                 }
                 if (best.feed_stage >= 0 && span_best < 0.99 * span_stream) {
-                    list_schedule(ss.data(), n, pairs, 2.0, off_s, ent_s, &span_stream, nullptr, &best);
+                    list_schedule(ss.data(), n, pairs, 2.0, off_s, ent_s, &span_stream, &best);
                     chosen = best;
                 }
             }

@@ -553,8 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_group_kernel(const GroupArgs g
 // ------------------------------------------------------------------ scheduling (host)
 
 void list_schedule(const SchedStage *st, int n, int units, double handoff, std::vector<int> &off,
-                   std::vector<WorkEntry> &entries, double *makespan, std::vector<double> *starts,
-                   const SchedOpts *opts)
+                   std::vector<WorkEntry> &entries, double *makespan, const SchedOpts *opts)
 {
     SchedOpts o;
     if (opts) o = *opts;
@@ -608,7 +607,6 @@ void list_schedule(const SchedStage *st, int n, int units, double handoff, std::
     // ---- placement: each tile to the allowed worker that can start it first
     std::vector<double> block_done(nblocks, 0.0);
     std::vector<std::vector<WorkEntry>> per(units);
-    std::vector<std::vector<double>> per_start(starts ? units : 0);
     // Small problems (one chain's few hundred tiles) or restricted workers: scan
     // the allowed workers, ties to the lowest index. Larger ones: a heap of (free
     // time, worker), O(log workers) per tile; a tile whose input is not ready
@@ -653,7 +651,6 @@ void list_schedule(const SchedStage *st, int n, int units, double handoff, std::
         else
             heap.push({fin, best});
         per[best].push_back(WorkEntry{(uint32_t)t.si, ((uint32_t)mb << 16) | (uint32_t)nb});
-        if (starts) per_start[best].push_back(start);
         double &bd = block_done[c.done_off + (c.row_done ? (long)nb * c.tiles_m + mb : nb)];
         if (fin > bd) bd = fin;
         if (fin > span) span = fin;
@@ -662,11 +659,9 @@ void list_schedule(const SchedStage *st, int n, int units, double handoff, std::
     off.assign(units + 1, 0);
     entries.clear();
     entries.reserve(total);
-    if (starts) starts->clear();
     for (int u = 0; u < units; ++u) {
         off[u + 1] = off[u] + (int)per[u].size();
         entries.insert(entries.end(), per[u].begin(), per[u].end());
-        if (starts) starts->insert(starts->end(), per_start[u].begin(), per_start[u].end());
     }
 }
 
@@ -710,6 +705,64 @@ cudaError_t single_capacity(int num_sms, int &ctas)
     }
     ctas = cap[dev & 63] * num_sms;  // num_sms may be fewer than the device's: a cap
     return cudaSuccess;
+}
+
+// The one list of a dynamic launch: every tile in order of an estimated start, each
+// dependency before its readers. A column block of a stage is the unit (its tiles share
+// their start): it starts once the block it reads is done, but not before the work
+// listed ahead of it would have occupied all units; stages in dependency depth order,
+// within a depth the ones with the longest path behind them first. The estimate costs a
+// few operations per block; placing every tile on its own worker gave the same device
+// times and took 370 us of host time for 4370 tiles, more than half of their run time.
+void dynamic_order(const SchedStage *st, int n, int units, double handoff, std::vector<WorkEntry> &entries)
+{
+    std::vector<int> depth(n, 0), order(n);
+    std::vector<double> behind(n, 0.0);  // the stages after this one, one tile each
+    long total = 0, nblocks = 0;
+    for (int i = 0; i < n; ++i) {
+        depth[i] = st[i].prev < 0 ? 0 : depth[st[i].prev] + 1;
+        order[i] = i;
+        total += (long)st[i].tiles_m * st[i].tiles_n;
+        nblocks += st[i].tiles_n;
+    }
+    for (int i = n - 1; i >= 0; --i)
+        if (st[i].prev >= 0)
+            behind[st[i].prev] = std::max(behind[st[i].prev], behind[i] + st[i].cost + handoff);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        return depth[x] != depth[y] ? depth[x] < depth[y] : behind[x] > behind[y];
+    });
+    struct Block {
+        double start;
+        int si, nb;
+    };
+    std::vector<Block> blocks;
+    blocks.reserve(nblocks);
+    std::vector<int> first(n);  // stage's first column block in `done`
+    int off = 0;
+    for (int i = 0; i < n; ++i) {
+        first[i] = off;
+        off += st[i].tiles_n;
+    }
+    std::vector<double> done(off, 0.0);
+    double work = 0.0;
+    for (int si : order) {
+        const SchedStage &c = st[si];
+        const double span = c.cost * std::max(1.0, (double)c.tiles_m / units);
+        for (int nb = 0; nb < c.tiles_n; ++nb) {
+            const double ready = c.prev >= 0 ? done[first[c.prev] + nb] + handoff : 0.0;
+            const double start = std::max(ready, work / units);
+            blocks.push_back(Block{start, si, nb});
+            done[first[si] + nb] = start + span;
+            work += c.cost * c.tiles_m;
+        }
+    }
+    std::stable_sort(blocks.begin(), blocks.end(),
+                     [](const Block &x, const Block &y) { return x.start < y.start; });
+    entries.clear();
+    entries.reserve(total);
+    for (const Block &b : blocks)
+        for (int mb = 0; mb < st[b.si].tiles_m; ++mb)
+            entries.push_back(WorkEntry{(uint32_t)b.si, ((uint32_t)mb << 16) | (uint32_t)b.nb});
 }
 
 template <int OP, int BN, int S>
@@ -780,21 +833,13 @@ cudaError_t plan_single(const StageArgs *stages, const int *prev, int n, int ker
     if (items < ctas) ctas = (int)items;
     std::vector<int> off;
     std::vector<WorkEntry> ent;
-    std::vector<double> starts;
     const bool dyn = group_dynamic();
-    list_schedule(ss.data(), n, ctas, 2.0, off, ent, nullptr, dyn ? &starts : nullptr);
     if (dyn) {
-        // one list in order of the schedule's start times (every dependency
-        // starts earlier, so it comes first), taken by the CTAs in turn
-        std::vector<int> order(ent.size());
-        for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
-        std::stable_sort(order.begin(), order.end(),
-                         [&](int x, int y) { return starts[x] < starts[y]; });
-        std::vector<WorkEntry> sorted(ent.size());
-        for (size_t i = 0; i < order.size(); ++i) sorted[i] = ent[order[i]];
-        ent.swap(sorted);
+        dynamic_order(ss.data(), n, ctas, 2.0, ent);
         off.assign(ctas + 1, (int)items);
         off[0] = 0;
+    } else {
+        list_schedule(ss.data(), n, ctas, 2.0, off, ent);
     }
     auto r = [](size_t b) { return (b + 255) & ~(size_t)255; };
     out.kernel = kernel;
@@ -830,8 +875,11 @@ cudaError_t launch_single(const GroupLaunch &g, const void *tables_dev, int *don
     a.next = done + g.done_ints - 1;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;  // all CTAs resident: they wait on one another
-    attr[0].val.cooperative = 1;
+    // static lists: all CTAs resident, since they wait on one another. A CTA that takes
+    // its tiles in turn waits only for tiles that running CTAs have taken, so that such
+    // grids may share the device with others.
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = g.dynamic ? 0 : 1;
     cfg.gridDim = dim3(g.ctas);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = G::SMEM_BYTES;

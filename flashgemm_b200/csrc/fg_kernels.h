@@ -101,7 +101,6 @@ struct SchedStage {
 // Worker u runs entries[off[u] .. off[u+1]) in that order, so the earliest
 // unfinished entry always heads its worker's list and no worker waits forever.
 // makespan (optional): the estimated finish time of the last tile.
-// starts (optional): each entry's estimated start, in the order of `entries`.
 //
 // Options (optional argument):
 // * feeders: the last `feed_workers` workers take the last `feed_rows` row
@@ -125,7 +124,7 @@ struct SchedOpts {
 };
 void list_schedule(const SchedStage *st, int n, int units, double handoff, std::vector<int> &off,
                    std::vector<WorkEntry> &entries, double *makespan = nullptr,
-                   std::vector<double> *starts = nullptr, const SchedOpts *opts = nullptr);
+                   const SchedOpts *opts = nullptr);
 
 enum GroupKernel : int {
     GK_PAIR = 0,        // BF16 / INT8: CTA pairs, 256 x 256 tiles, 6-stage ring
