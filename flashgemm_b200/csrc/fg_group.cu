@@ -667,9 +667,6 @@ void list_schedule(const SchedStage *st, int n, int units, double handoff, std::
 
 // ------------------------------------------------------------------ planning and launch (host)
 
-namespace {
-
-// Dynamic lists for the single-CTA kernel (FG_GROUP_DYNAMIC=0: static per-CTA lists).
 bool group_dynamic()
 {
     static const bool on = [] {
@@ -678,6 +675,8 @@ bool group_dynamic()
     }();
     return on;
 }
+
+namespace {
 
 template <int OP, int BN, int S>
 cudaError_t single_capacity(int num_sms, int &ctas)

@@ -146,6 +146,9 @@ struct GroupLaunch {
     std::vector<unsigned char> tables;
 };
 
+// Dynamic lists for the single-CTA kernel (FG_GROUP_DYNAMIC=0: static per-CTA lists).
+bool group_dynamic();
+
 // Column width of a kernel's tiles (the unit of its dependency counters).
 int group_tile_n(int kernel, int op);
 cudaError_t plan_group(const StageArgs *stages, const int *prev, int n, int kernel, int num_sms,

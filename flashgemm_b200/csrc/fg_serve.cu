@@ -39,15 +39,19 @@ struct fg_server_s {
         std::vector<GroupExec> gx;  // host tables, kept until the batch completes
         int slot = 0;
         size_t bytes = 0;
-        void *mem = nullptr, *tab = nullptr;
+        void *mem = nullptr;
+        void *tab[3] = {nullptr, nullptr, nullptr};  // grouped tables per dtype
         int status = FG_OK;
     };
 
     DevCtx *c = nullptr;
     fg_server_opts o{};
     cudaMemPool_t pool = nullptr;
-    std::vector<cudaStream_t> streams;
-    std::vector<cudaEvent_t> events;
+    std::vector<cudaStream_t> streams;  // per slot: copies, and one dtype's launches
+    std::vector<cudaStream_t> sides;    // two per slot: the other dtypes' launches
+    std::vector<cudaEvent_t> events;    // per slot: the batch is done
+    std::vector<cudaEvent_t> forks;     // two per slot: a side stream may start / has ended
+    bool cap_given = false;             // ctas_per_batch was set by the caller
     int *status_dev = nullptr;   // one word per slot
     int *status_host = nullptr;  // pinned copies
 
@@ -116,9 +120,14 @@ void server_finish(fg_server_s *s, fg_server_s::Batch *b, double t)
     s->free_slots.push_back(b->slot);
 }
 
-// Launches one batch on its slot's stream: device copies of host operands,
-// one grouped launch per dtype present, copies of host results, an event.
-int server_launch(fg_server_s *s, fg_server_s::Batch *b)
+// Launches one batch: device copies of host operands on its slot's stream, one grouped
+// launch per dtype present, each as soon as the host has built it and on a stream of its
+// own (one dtype's last tiles leave SMs that the next one's first take), copies of host
+// results, an event. alone: no other batch is in flight, so that kernels whose CTAs wait
+// on no CTA still to be started may take every SM; others keep to the batch's cap.
+// Measured (B200, burst of 48 mixed requests): all built, then launched in turn on half the
+// SMs each 1192 us, so 1040; with placing per tile before that 2280.
+int server_launch(fg_server_s *s, fg_server_s::Batch *b, bool alone)
 {
     DevCtx *c = s->c;
     const int slot = b->slot;
@@ -148,38 +157,57 @@ int server_launch(fg_server_s *s, fg_server_s::Batch *b)
             dC[i] = r.C;
         }
     }
-    // one grouped launch per dtype
-    size_t tab_total = 0;
-    std::vector<std::vector<fg_chain_desc>> per(3);
-    const int dts[3] = {FG_DT_BF16, FG_DT_INT8, FG_DT_F32};
+    // one grouped launch per dtype, the one with the most work first
+    struct Part {
+        int dtype;
+        std::vector<fg_chain_desc> chains;
+        double flops = 0.0;
+    };
+    Part per[3];
+    per[0].dtype = FG_DT_BF16;
+    per[1].dtype = FG_DT_INT8;
+    per[2].dtype = FG_DT_F32;
     for (size_t i = 0; i < b->reqs.size(); ++i) {
         const fg_request &r = b->reqs[i]->r;
-        for (int d = 0; d < 3; ++d)
-            if (r.dtype == dts[d])
-                per[d].push_back(fg_chain_desc{dC[i], dB[i], r.N, r.num_gemm, r.W});
+        for (Part &p : per)
+            if (r.dtype == p.dtype) {
+                p.chains.push_back(fg_chain_desc{dC[i], dB[i], r.N, r.num_gemm, r.W});
+                p.flops += b->reqs[i]->flops;
+            }
     }
+    std::stable_sort(per, per + 3, [](const Part &x, const Part &y) { return x.flops > y.flops; });
     b->gx.resize(3);
-    const int cap = s->o.ctas_per_batch;
+    int launched = 0;
     for (int d = 0; d < 3; ++d) {
-        if (per[d].empty()) continue;
-        const int a = dts[d] == FG_DT_F32 ? algo : 0;
+        if (per[d].chains.empty()) continue;
+        const int dtype = per[d].dtype, n = (int)per[d].chains.size();
+        const int a = dtype == FG_DT_F32 ? algo : 0;
         int kernel = g_group_kernel.load(), order = g_group_order.load();
-        group_resolve(c, dts[d], a, (int)per[d].size(), per[d].data(), kernel, order);
-        int e = group_build(c, dts[d], a, kernel, order, (int)per[d].size(), per[d].data(), cv,
-                            b->gx[d], status, cap);
+        group_resolve(c, dtype, a, n, per[d].chains.data(), kernel, order);
+        const bool all_sms = alone && !s->cap_given && kernel != GK_PAIR && group_dynamic();
+        int e = group_build(c, dtype, a, kernel, order, n, per[d].chains.data(), cv, b->gx[d], status,
+                            all_sms ? c->sms : s->o.ctas_per_batch);
         if (e) return e;
-        tab_total += group_tab_bytes(b->gx[d]);
-    }
-    if (cv.off > b->bytes) return fail(FG_ERR_NOMEM, "serving: admission estimate too small");
-    CUDA_TRY(cudaMallocFromPoolAsync(&b->tab, tab_total, s->pool, st));
-    Carver ct;
-    ct.base = (char *)b->tab;
-    for (int d = 0; d < 3; ++d) {
-        if (per[d].empty()) continue;
+        if (cv.off > b->bytes) return fail(FG_ERR_NOMEM, "serving: admission estimate too small");
+        CUDA_TRY(cudaMallocFromPoolAsync(&b->tab[d], group_tab_bytes(b->gx[d]), s->pool, st));
+        Carver ct;
+        ct.base = (char *)b->tab[d];
         group_place(b->gx[d], ct);
-        int e = group_upload(b->gx[d], st, false);
-        if (e) return e;
-        if ((e = group_launch(c, b->gx[d], st, false, status))) return e;
+        cudaStream_t on = st;
+        if (launched > 0) {
+            on = s->sides[2 * slot + launched - 1];
+            cudaEvent_t ev = s->forks[2 * slot + launched - 1];
+            CUDA_TRY(cudaEventRecord(ev, st));  // operands and tables are there
+            CUDA_TRY(cudaStreamWaitEvent(on, ev, 0));
+        }
+        ++launched;
+        if ((e = group_upload(b->gx[d], on, false))) return e;
+        if ((e = group_launch(c, b->gx[d], on, false, status))) return e;
+    }
+    for (int i = 1; i < launched; ++i) {  // the slot's stream goes on after all of them
+        cudaEvent_t ev = s->forks[2 * slot + i - 1];
+        CUDA_TRY(cudaEventRecord(ev, s->sides[2 * slot + i - 1]));
+        CUDA_TRY(cudaStreamWaitEvent(st, ev, 0));
     }
     for (size_t i = 0; i < b->reqs.size(); ++i) {
         const fg_request &r = b->reqs[i]->r;
@@ -192,7 +220,8 @@ int server_launch(fg_server_s *s, fg_server_s::Batch *b)
             CUDA_TRY(cudaMemcpyAsync(r.C, dC[i], (size_t)rows * r.N * 4, cudaMemcpyDeviceToHost, st));
     }
     CUDA_TRY(cudaMemcpyAsync(s->status_host + slot, status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaFreeAsync(b->tab, st));
+    for (void *t : b->tab)
+        if (t) CUDA_TRY(cudaFreeAsync(t, st));
     CUDA_TRY(cudaFreeAsync(b->mem, st));
     CUDA_TRY(cudaEventRecord(s->events[slot], st));
     return FG_OK;
@@ -267,16 +296,19 @@ void server_dispatch_loop(fg_server_s *s)
         s->peak = std::max(s->peak, s->used);
         ++s->batches;
         s->batched += (long long)b->reqs.size();
+        const bool alone = s->inflight.empty();
         lk.unlock();
         int st;
         {
             std::lock_guard<std::mutex> g(s->c->mu);
-            st = server_launch(s, b);
+            st = server_launch(s, b, alone);
         }
         if (st) {  // nothing more runs for this batch: return its memory to the pool
             cudaGetLastError();
             cudaStream_t bs = s->streams[b->slot];
-            if (b->tab) cudaFreeAsync(b->tab, bs);
+            for (int i = 0; i < 2; ++i) cudaStreamSynchronize(s->sides[2 * b->slot + i]);
+            for (void *t : b->tab)
+                if (t) cudaFreeAsync(t, bs);
             if (b->mem) cudaFreeAsync(b->mem, bs);
             cudaStreamSynchronize(bs);
             cudaGetLastError();
@@ -333,6 +365,7 @@ FG_EXPORT int fg_server_create(const fg_server_opts *opts, fg_server *out)
     if (s->o.slots <= 0) s->o.slots = 2;
     if (s->o.slots > 16) s->o.slots = 16;
     if (s->o.max_wait_us <= 0) s->o.max_wait_us = 200;
+    s->cap_given = s->o.ctas_per_batch > 0;
     if (s->o.ctas_per_batch <= 0) s->o.ctas_per_batch = std::max(2, c->sms / s->o.slots);
     if (s->o.hbm_budget <= 0) {
         size_t fr = 0, tot = 0;
@@ -348,6 +381,12 @@ FG_EXPORT int fg_server_create(const fg_server_opts *opts, fg_server *out)
     CUDA_TRY(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     s->streams.resize(s->o.slots);
     s->events.resize(s->o.slots);
+    s->sides.resize(2 * s->o.slots);
+    s->forks.resize(2 * s->o.slots);
+    for (int i = 0; i < 2 * s->o.slots; ++i) {
+        CUDA_TRY(cudaStreamCreateWithFlags(&s->sides[i], cudaStreamNonBlocking));
+        CUDA_TRY(cudaEventCreateWithFlags(&s->forks[i], cudaEventDisableTiming));
+    }
     for (int i = 0; i < s->o.slots; ++i) {
         CUDA_TRY(cudaStreamCreateWithFlags(&s->streams[i], cudaStreamNonBlocking));
         CUDA_TRY(cudaEventCreateWithFlags(&s->events[i], cudaEventDisableTiming));
@@ -511,7 +550,9 @@ FG_EXPORT int fg_server_destroy(fg_server s)
         cudaStreamSynchronize(st);
         cudaStreamDestroy(st);
     }
+    for (auto st : s->sides) cudaStreamDestroy(st);
     for (auto e : s->events) cudaEventDestroy(e);
+    for (auto e : s->forks) cudaEventDestroy(e);
     cudaFree(s->status_dev);
     cudaFreeHost(s->status_host);
     cudaMemPoolDestroy(s->pool);

@@ -203,8 +203,10 @@ int fg_group_choice(int dtype, int nchains, const fg_chain_desc *chains, int *ke
  * weights are admitted in arrival order while the device-memory budget and a
  * launch slot allow, packed into grouped launches (one per dtype present) and
  * run on one of `slots` streams, so a batch admitted while others are still on
- * the GPU overlaps with them (each batch's persistent grid is capped at
- * SMs / slots CTAs unless ctas_per_batch says otherwise). The device is never
+ * the GPU overlaps with them (each batch's persistent grids are capped at
+ * SMs / slots CTAs unless ctas_per_batch says otherwise; a batch launched while
+ * none is in flight may take every SM, and one that follows starts as its CTAs
+ * leave). The device is never
  * left idle while requests wait: a batch is launched at once when no other is
  * in flight, else when it holds max_batch requests or its oldest request has
  * waited max_wait_us. Results are the ones fg_chain_registered gives for the
