@@ -77,6 +77,8 @@ __device__ __forceinline__ void split_rows(const SplitJob &j, long part, long pa
 // device memory.
 __global__ void __launch_bounds__(256) split_tf32_kernel(const __grid_constant__ SplitBatch b)
 {
+    overlap_next();
+    overlap_wait();
     split_rows(b.job[blockIdx.y], blockIdx.x, gridDim.x);
 }
 __global__ void __launch_bounds__(256) split_tf32_jobs_kernel(const SplitJob *__restrict__ jobs)
@@ -101,8 +103,7 @@ cudaError_t launch_split_tf32(const SplitBatch &b, cudaStream_t s)
         most = e > most ? e : most;
     }
     if (most < 1) return cudaSuccess;
-    split_tf32_kernel<<<dim3(split_blocks(most), (unsigned)b.n), 256, 0, s>>>(b);
-    return cudaGetLastError();
+    return launch_overlapped(split_tf32_kernel, dim3(split_blocks(most), (unsigned)b.n), 256, 0, s, b);
 }
 
 cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long max_elems,
@@ -170,8 +171,10 @@ cudaError_t launch_prep_int8_weights(const int8_t *src, long ld_in, uint8_t *dst
 }
 
 // Several preparations in one launch (blockIdx.y = job).
-__global__ void prep_int8_jobs_kernel(const PrepJob *__restrict__ jobs_unused, PrepJobs jobs)
+__global__ void prep_int8_jobs_kernel(const __grid_constant__ PrepJobs jobs)
 {
+    overlap_next();
+    overlap_wait();
     const PrepJob &j = jobs.job[blockIdx.y];
     const long per_row = j.ld_out / 16;
     const long total = j.M * per_row;
@@ -216,8 +219,7 @@ cudaError_t launch_prep_int8_jobs(const PrepJobs &jobs, cudaStream_t s)
     long blocks = (most + 255) / 256;
     if (blocks > 148 * 4) blocks = 148 * 4;
     if (blocks < 1) blocks = 1;
-    prep_int8_jobs_kernel<<<dim3((unsigned)blocks, jobs.n), 256, 0, s>>>(nullptr, jobs);
-    return cudaGetLastError();
+    return launch_overlapped(prep_int8_jobs_kernel, dim3((unsigned)blocks, jobs.n), 256, 0, s, jobs);
 }
 
 __global__ void fill_u32_kernel(uint32_t *dst, size_t count, uint32_t value)

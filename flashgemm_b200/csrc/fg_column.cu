@@ -176,6 +176,7 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
         fence_mbar_init();
         // the ring's first round needs no wait, and nobody else: under way before the
         // CTA meets, and before the later stages' tensor maps are fetched
+        overlap_wait();
         for (int kb = 0; kb < first_loads; ++kb)
             load(0, blockIdx.x, 0, kb, kb, (kb / chunk_blocks(0)) & 1);
         for (int i = 1; i < g.n; ++i) {
@@ -188,6 +189,8 @@ __global__ void __launch_bounds__(c_threads(EW), PER) tc_column_kernel(const __g
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
+    overlap_next();
+    overlap_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -690,11 +693,10 @@ cudaError_t launch_column(const PanelChainArgs &a, int num_sms, int *status, cud
         g = hit->g;  // a copy: the entry may go once the lock is released
     }
     const int grid = std::min(g.nblocks, num_sms * (g.small ? 2 : 1));
-    if (g.small)
-        tc_column_kernel<kCSmallRows / 16, 4, 2><<<grid, c_threads(4), g.smem, s>>>(g);
-    else
-        tc_column_kernel<(kCRows / 16 + 1) / 2, 8, 1><<<grid, c_threads(8), g.smem, s>>>(g);
-    return cudaGetLastError();
+    return g.small ? launch_overlapped(tc_column_kernel<kCSmallRows / 16, 4, 2>, dim3(grid), c_threads(4),
+                                       g.smem, s, g)
+                   : launch_overlapped(tc_column_kernel<(kCRows / 16 + 1) / 2, 8, 1>, dim3(grid),
+                                       c_threads(8), g.smem, s, g);
 }
 
 }  // namespace fg

@@ -242,6 +242,8 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
+    overlap_next();
+    overlap_wait();
 
     NarrowWalk walk;
     walk.init(g);
@@ -754,18 +756,10 @@ int narrow_units_per_cta(const NarrowArgs &P, int grid)
 cudaError_t launch_narrow(NarrowArgs &P, int grid, int *status, cudaStream_t s)
 {
     P.status = status;
-    if (P.op == OP_BF16) {
-        if (P.epi_warps == 8)
-            tc_narrow_kernel<OP_BF16, 8><<<grid, n_threads(8), P.smem, s>>>(P);
-        else
-            tc_narrow_kernel<OP_BF16, 4><<<grid, n_threads(4), P.smem, s>>>(P);
-    } else {
-        if (P.epi_warps == 8)
-            tc_narrow_kernel<OP_I8, 8><<<grid, n_threads(8), P.smem, s>>>(P);
-        else
-            tc_narrow_kernel<OP_I8, 4><<<grid, n_threads(4), P.smem, s>>>(P);
-    }
-    return cudaGetLastError();
+    const bool wide = P.epi_warps == 8;
+    auto *kernel = P.op == OP_BF16 ? (wide ? tc_narrow_kernel<OP_BF16, 8> : tc_narrow_kernel<OP_BF16, 4>)
+                                   : (wide ? tc_narrow_kernel<OP_I8, 8> : tc_narrow_kernel<OP_I8, 4>);
+    return launch_overlapped(kernel, dim3(grid), n_threads(P.epi_warps), P.smem, s, P);
 }
 
 }  // namespace fg

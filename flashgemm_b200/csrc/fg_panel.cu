@@ -233,6 +233,8 @@ __global__ void __launch_bounds__(kPThreads, 1) tc_panel_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = bars->tmem_base;
+    overlap_next();
+    overlap_wait();
 
     TileWalk walk;
     walk.init(g, blockIdx.x);
@@ -709,8 +711,7 @@ cudaError_t launch_panel_one(const PanelChainArgs &a, int num_sms, int *status, 
     }
     g.trace = trace;
     const int grid = std::min(g.one_blocks, ctas);
-    tc_panel_kernel<<<grid, kPThreads, kPSmem, s>>>(g);
-    return cudaGetLastError();
+    return launch_overlapped(tc_panel_kernel, dim3(grid), kPThreads, kPSmem, s, g);
 }
 
 }  // namespace fg
