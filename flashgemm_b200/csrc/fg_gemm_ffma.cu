@@ -29,7 +29,8 @@
 // reads), pairs along the diagonal (no faster), scalar FMAs (0.9x), registers
 // between global and shared memory instead of cp.async (the kernel before this
 // one). Before and now, us a call (B200): 1024^3 79 -> 58 (27 -> 37 TFLOP/s),
-// 1632 x 36548 x 1024 2693 -> 2409 (51 TFLOP/s), 35 x 8457 x 2560 141 -> 99.
+// 1632 x 36548 x 1024 2693 -> 2410 (51 TFLOP/s), 35 x 8457 x 2560 141 -> 86,
+// 512 x 289 x 1024 65 -> 29, 4096^3 3577 -> 2588.
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -79,9 +80,10 @@ __device__ __forceinline__ void copy_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int BM_, int BN_, int BK_, int TM_, int TN_, int ST_>
+template <int BM_, int BN_, int BK_, int TM_, int TN_, int ST_, int OCC_>
 struct Shape {
     static constexpr int BM = BM_, BN = BN_, BK = BK_, TM = TM_, TN = TN_, ST = ST_;
+    static constexpr int OCC = OCC_;  // CTAs per SM: what the registers have to allow
     static constexpr int TX = BN / TN, TY = BM / TM, NT = TX * TY;
     static constexpr int STAGE = (BM + BN) * BK;  // floats per ring buffer
     static constexpr int SMEM = ST * STAGE * 4;
@@ -300,17 +302,18 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
     }
 }
 
-// m_fast: neighbouring CTAs share columns of B rather than rows of A. With p.part,
-// blockIdx.z is a K block of its own: block 0 writes C, block z part z - 1, for
-// ffma_add_blocks_kernel.
-template <class S, bool VA, bool VB>
-__global__ void __launch_bounds__(S::NT) ffma_sgemm_kernel(FfmaArgs p, int tiles_m, int tiles_n,
+// m_fast: neighbouring CTAs share columns of B rather than rows of A. APART (p.part is
+// set): blockIdx.z is a K block of its own; block 0 writes C, block z part z - 1, for
+// ffma_add_blocks_kernel. (A kernel of its own: arguments that change live in registers,
+// which costs the other one 5 %.)
+template <class S, bool VA, bool VB, bool APART>
+__global__ void __launch_bounds__(S::NT, S::OCC) ffma_sgemm_kernel(FfmaArgs p, int tiles_m, int tiles_n,
                                                            int m_fast)
 {
     extern __shared__ __align__(128) float sm[];
     const int t = blockIdx.x;
     const int tm = m_fast ? t % tiles_m : t / tiles_n, tn = m_fast ? t / tiles_m : t % tiles_n;
-    if (p.part) {
+    if constexpr (APART) {
         const int z = blockIdx.z, k0 = z * p.kblock;
         p.A += k0;
         p.B += (size_t)k0 * p.ldb;
@@ -330,6 +333,8 @@ __global__ void __launch_bounds__(S::NT) ffma_sgemm_kernel(FfmaArgs p, int tiles
 template <bool VEC>
 __global__ void __launch_bounds__(256) ffma_add_blocks_kernel(const FfmaArgs p, int parts)
 {
+    overlap_next();
+    overlap_wait();
     const long quads = (p.N + 3) / 4, total = quads * p.M;
     const size_t step = (size_t)p.M * p.ld_part;
     for (long i = blockIdx.x * 256l + threadIdx.x; i < total; i += gridDim.x * 256l) {
@@ -361,7 +366,7 @@ __global__ void __launch_bounds__(256) ffma_add_blocks_kernel(const FfmaArgs p, 
 
 // Many independent SGEMMs: CTA b works on job j with tile0[j] <= b < tile0[j + 1].
 template <class S>
-__global__ void __launch_bounds__(S::NT) ffma_group_kernel(const FfmaJob *__restrict__ jobs, int njobs)
+__global__ void __launch_bounds__(S::NT, S::OCC) ffma_group_kernel(const FfmaJob *__restrict__ jobs, int njobs)
 {
     extern __shared__ __align__(128) float sm[];
     const int b = blockIdx.x;
@@ -388,11 +393,11 @@ __global__ void __launch_bounds__(S::NT) ffma_group_kernel(const FfmaJob *__rest
         ffma_tile<S, false, false>(p, m0, n0, sm);
 }
 
-using Wide = Shape<64, 128, 32, 8, 8, 3>;
-using Square = Shape<64, 64, 32, 4, 8, 3>;
-using Low = Shape<40, 64, 32, 5, 4, 3>;
-using Small = Shape<32, 64, 32, 4, 4, 3>;
-using Tiny = Shape<16, 64, 32, 2, 4, 3>;
+using Wide = Shape<64, 128, 32, 8, 8, 3, 3>;
+using Square = Shape<64, 64, 32, 4, 8, 3, 4>;
+using Low = Shape<40, 64, 32, 5, 4, 3, 4>;
+using Small = Shape<32, 64, 32, 4, 4, 3, 4>;
+using Tiny = Shape<16, 64, 32, 2, 4, 3, 5>;
 
 // The tile shapes: CTAs resident per SM, and FMA per clock that an SM reaches with
 // one CTA and with all of them (B200; from 256 x 256 x 2048, which gives every shape
@@ -402,12 +407,12 @@ struct ShapeInfo {
     double one, full;
 };
 constexpr ShapeInfo kShapes[] = {
-    {64, 128, 3, 78.5, 87.9},   // Wide: the best rate; 128 x 128 (8 x 16 per thread) gains nothing on
+    {64, 128, Wide::OCC, 78.5, 87.9},   // Wide: the best rate; 128 x 128 (8 x 16 per thread) gains nothing on
                                 // it and leaves the SMs idle at both ends of a short K
-    {64, 64, 4, 61.0, 83.9},    // Square: two or three per SM where Wide leaves SMs idle
-    {40, 64, 4, 48.0, 79.8},    // Low: few rows, and dimensions that 64 pads
-    {32, 64, 4, 43.5, 72.7},    // Small: more CTAs where outputs are few
-    {16, 64, 5, 28.8, 40.0},    // Tiny: at most one CTA per SM
+    {64, 64, Square::OCC, 61.0, 83.9},    // Square: two or three per SM where Wide leaves SMs idle
+    {40, 64, Low::OCC, 48.0, 79.8},    // Low: few rows, and dimensions that 64 pads
+    {32, 64, Small::OCC, 43.5, 72.7},    // Small: more CTAs where outputs are few
+    {16, 64, Tiny::OCC, 28.8, 40.0},    // Tiny: at most one CTA per SM
 };
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
@@ -470,19 +475,25 @@ cudaError_t allow_smem(F *f, int smem, unsigned long long &done, std::mutex &mu)
     return e;
 }
 
-template <class S, bool VA, bool VB>
+template <class S, bool VA, bool VB, bool APART>
 cudaError_t launch_tiles(const FfmaArgs &a, cudaStream_t s)
 {
     static unsigned long long done;
     static std::mutex mu;
-    const cudaError_t e = allow_smem(ffma_sgemm_kernel<S, VA, VB>, S::SMEM, done, mu);
+    const cudaError_t e = allow_smem(ffma_sgemm_kernel<S, VA, VB, APART>, S::SMEM, done, mu);
     if (e != cudaSuccess) return e;
     const long tm = (a.M + S::BM - 1) / S::BM, tn = (a.N + S::BN - 1) / S::BN;
     if (tm * tn > 0x7fffffffl) return cudaErrorInvalidConfiguration;
-    const unsigned blocks = a.part ? (unsigned)((a.K + a.kblock - 1) / a.kblock) : 1u;
-    ffma_sgemm_kernel<S, VA, VB>
+    const unsigned blocks = APART ? (unsigned)((a.K + a.kblock - 1) / a.kblock) : 1u;
+    ffma_sgemm_kernel<S, VA, VB, APART>
         <<<dim3((unsigned)(tm * tn), 1, blocks), S::NT, S::SMEM, s>>>(a, (int)tm, (int)tn, tm <= tn);
     return cudaGetLastError();
+}
+
+template <class S, bool VA, bool VB>
+cudaError_t launch_apart(const FfmaArgs &a, cudaStream_t s)
+{
+    return a.part ? launch_tiles<S, VA, VB, true>(a, s) : launch_tiles<S, VA, VB, false>(a, s);
 }
 
 template <class S>
@@ -490,8 +501,8 @@ cudaError_t launch_shape(const FfmaArgs &a, cudaStream_t s)
 {
     const bool va = a.lda % 4 == 0 && ((uintptr_t)a.A & 15) == 0;
     const bool vb = a.ldb % 4 == 0 && ((uintptr_t)a.B & 15) == 0;
-    if (va) return vb ? launch_tiles<S, true, true>(a, s) : launch_tiles<S, true, false>(a, s);
-    return vb ? launch_tiles<S, false, true>(a, s) : launch_tiles<S, false, false>(a, s);
+    if (va) return vb ? launch_apart<S, true, true>(a, s) : launch_apart<S, true, false>(a, s);
+    return vb ? launch_apart<S, false, true>(a, s) : launch_apart<S, false, false>(a, s);
 }
 
 }  // namespace
@@ -524,9 +535,9 @@ cudaError_t launch_ffma_group(const FfmaJob *jobs_dev, int njobs, int total_tile
 // SMs idle they run side by side, the sums of all but the first in a workspace, and
 // a second kernel adds them in order: the same bits. That costs the launch (about
 // 3 us) and the parts' traffic; it is taken where the tiles' cost falls by more.
-// Measured (B200, us a call; first figure: this tile, blocks in turn): 35 x 8457 x 2560
-// 99 -> 92, 128 x 2048 x 4096 98 -> 76 (the kernel before this tile: 278),
-// 1024 x 16 x 500000 1468 (38000 before).
+// Measured (B200, us a call; first figure: the kernel before this tile, which could not):
+// 128 x 2048 x 4096 276 -> 72, 84 x 1024 x 4096 303 -> 45, 35 x 8457 x 2560 141 -> 86,
+// 1024 x 16 x 500000 38000 -> 1436.
 size_t ffma_sgemm_workspace(long M, long N, long K, int kblock, int num_sms)
 {
     if (M <= 0 || N <= 0 || kblock <= 0 || K <= kblock) return 0;
@@ -562,11 +573,9 @@ cudaError_t launch_ffma_sgemm(const FfmaArgs &a, int num_sms, cudaStream_t s)
     const int parts = (a.K + a.kblock - 1) / a.kblock - 1;
     const long ctas = ((a.N + 3) / 4 * (long)a.M + 255) / 256;
     const unsigned grid = (unsigned)(ctas < num_sms * 8l ? ctas : num_sms * 8l);
-    if (a.ldc % 4 == 0 && ((uintptr_t)a.C & 15) == 0)
-        ffma_add_blocks_kernel<true><<<grid, 256, 0, s>>>(a, parts);
-    else
-        ffma_add_blocks_kernel<false><<<grid, 256, 0, s>>>(a, parts);
-    return cudaGetLastError();
+    return launch_overlapped(a.ldc % 4 == 0 && ((uintptr_t)a.C & 15) == 0 ? ffma_add_blocks_kernel<true>
+                                                                          : ffma_add_blocks_kernel<false>,
+                             dim3(grid), 256, 0, s, a, parts);
 }
 
 }  // namespace fg
