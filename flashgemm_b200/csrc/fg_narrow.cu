@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <memory>
@@ -578,19 +579,6 @@ bool narrow_eligible(const StageArgs *st, int n)
     return true;
 }
 
-// On B200, over the reference's chain table (N 3136..65536, K_1 288..4800):
-// INT8 chains run faster narrow at every width (their fused path pays the
-// tail-row preparation and an int8 round trip per stage); BF16 chains whose
-// 128-column blocks fill fewer than half the SMs run their deep first stage on
-// too few SMs and are faster on the fused chain kernel, which splits rows too.
-bool narrow_preferred(const StageArgs *st, int n, int num_sms)
-{
-    (void)n;
-    if (st[0].op == OP_I8) return true;
-    const long nblk = (st[0].N + kNBN - 1) / kNBN;
-    return 2 * nblk >= num_sms;
-}
-
 namespace {
 
 // The shared memory layout of a chain: the weight boxes of the widest unit
@@ -635,6 +623,46 @@ bool narrow_layout(const StageArgs *st, int n, NarrowArgs &A)
     }
     return false;
 }
+
+}  // namespace
+
+// Microseconds of both kernels, fitted to measurements on B200 of 15 chains (64,64,64 to
+// 4800,192,56,336 and 64,128,4096) at N = 64 to 65536, registered weights, both types.
+// Narrow: a block's stages one after the other (per stage, per k-block, per row tile of
+// the last stage), the blocks of one SM in turn, half hidden where two are in flight.
+// Fused: a stage's tiles over all CTA pairs. Measured, us, narrow / fused: BF16 64,64,64
+// at N = 64 10 / 12, 1296,144,32,192 at 16384 22 / 27 but at 20000 (two rounds of blocks)
+// 41 / 35, 64,128,4096 at 64 57 / 12; INT8 4800,192,56,336 at 4096 32 / 41, 64,128,4096
+// at 1024 68 / 33.
+bool narrow_preferred(const StageArgs *st, int n, int num_sms)
+{
+    static thread_local NarrowArgs A;
+    const bool i8 = st[0].op == OP_I8;
+    if (!(i8 ? narrow_layout<OP_I8>(st, n, A) : narrow_layout<OP_BF16>(st, n, A))) return false;
+    const double kb_elems = i8 ? 128.0 : 64.0;
+    const long N = st[0].N, pairs = num_sms / 2;
+    double block = i8 ? 6.0 : 5.0, fused = 8.0;
+    bool tails = false;
+    for (int i = 0; i < n; ++i) {
+        const double kb = std::ceil(st[i].K / kb_elems);
+        const int rt = (st[i].M + 127) / 128;
+        if (i + 1 < n)
+            block += 1.2 + kb * (rt == 1 ? (i8 ? 0.22 : 0.24) : (i8 ? 0.35 : 0.42));
+        else
+            block += rt * (i8 ? 1.9 + 0.2 * kb : 1.0 + 0.25 * kb);
+        const double rounds =
+            std::ceil((double)((st[i].M + 255) / 256) * ((N + 255) / 256) / pairs);
+        fused += 3.4 + kb * rounds * (i8 ? 0.25 : 0.3) + (rounds - 1.0) * (i8 ? 4.0 : 3.0);
+        tails = tails || st[i].tail_hi > st[i].tail_lo;
+    }
+    if (tails) fused += 14.0;  // the fused kernel reads each tail row's quad per tile
+    const double rounds = std::ceil((double)((N + kNBN - 1) / kNBN) / num_sms);
+    const double narrow =
+        3.0 + block + (rounds - 1.0) * block * (A.xslots > 1 ? 0.5 : 1.0) * (i8 ? 1.0 : 1.05);
+    return narrow < fused;
+}
+
+namespace {
 
 template <int OP>
 cudaError_t narrow_attr(int smem)

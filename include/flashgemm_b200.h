@@ -77,8 +77,9 @@ int fg_get_chain_mode(void);
  * them on chip (the narrow chain kernel: one CTA per 128-column block, each
  * intermediate narrowed and permuted straight into shared memory; same
  * results as the other paths).
- * FG_NARROW_AUTO (default): where it is measured faster: every INT8 chain, and
- *   BF16 chains with at least one 128-column block per two SMs.
+ * FG_NARROW_AUTO (default): where a model fitted to measurements expects it to be
+ *   faster (most chains but those with a wide last stage or a deep first stage
+ *   on few columns).
  * FG_NARROW_ALWAYS: every such chain.  FG_NARROW_OFF: never.
  * The environment variable FG_NARROW (0 / 1 / auto) sets the initial mode. */
 enum { FG_NARROW_OFF = 0, FG_NARROW_ALWAYS = 1, FG_NARROW_AUTO = 2 };
