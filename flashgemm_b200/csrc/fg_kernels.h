@@ -213,13 +213,15 @@ cudaError_t launch_single_group(const GroupLaunch &g, const void *tables_dev, in
 
 constexpr int kNarrowRows = 256;
 constexpr int kNarrowMaxStages = 8;
-constexpr int kNarrowMaxRing = 4;
+constexpr int kNarrowMaxRing = 8;
 constexpr int kNarrowMaxX = 4;       // column blocks in flight per CTA, at most
 
 struct alignas(64) NarrowStage {
-    CUtensorMap tm_w;    // weights, K-major boxes of 128 rows x 128 bytes
-    CUtensorMap tm_wt;   // INT8 reference tail block (else = tm_w)
-    CUtensorMap tm_out;  // last stage: the result (staged TMA stores)
+    // weights, K-major boxes of 128-byte rows, of `box` rows for row tiles 0 and 1 of an
+    // intermediate (the last stage: 0 for all of its tiles)
+    CUtensorMap tm_w[2];
+    CUtensorMap tm_wt;   // INT8 reference tail block, for the one row tile that holds it
+    int box[2];
     int M, K;
     int permute;         // the reference's panel permutation between stages
     int tail_lo, tail_hi, tail_row0;
@@ -231,14 +233,15 @@ struct alignas(64) NarrowStage {
 struct alignas(64) NarrowArgs {
     NarrowStage st[kNarrowMaxStages];
     CUtensorMap tm_b;    // first stage's activations (K_1 x N), MN-major boxes
+    CUtensorMap tm_out;  // last stage: the result (staged TMA stores)
     const void *b;       // the same, for the INT8 tail correction
     long ldb;
     int n, N, nblocks;
     int op;              // OperandKind
-    // shared memory layout of the launch: ring slots of slot_bytes (ra weight
-    // boxes, then the first stage's activation boxes), xslots operand buffers
+    // shared memory layout of the launch: ring slots of slot_bytes (a unit's weight
+    // boxes, then at b_off the first stage's activation boxes), xslots operand buffers
     // of x_bytes (one per column block in flight, 1 to kNarrowMaxX), smem bytes in all
-    int ring, slot_bytes, ra, x_bytes, xslots, smem;
+    int ring, slot_bytes, b_off, x_bytes, xslots, smem;
     int epi_warps;       // 4 or 8 epilogue warps
     int *status;
     // optional (else null): kNarrowTraceFields %globaltimer stamps per (CTA, unit)

@@ -233,10 +233,11 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
         // the tensor maps into the TMA unit's cache before their first use
         tma_prefetch_desc(&g.tm_b);
         for (int i = 0; i < g.n; ++i) {
-            tma_prefetch_desc(&g.st[i].tm_w);
+            tma_prefetch_desc(&g.st[i].tm_w[0]);
             if (g.st[i].tail_hi > g.st[i].tail_lo) tma_prefetch_desc(&g.st[i].tm_wt);
+            if (g.st[i].box[1] && g.st[i].box[1] != g.st[i].box[0]) tma_prefetch_desc(&g.st[i].tm_w[1]);
         }
-        tma_prefetch_desc(&g.st[g.n - 1].tm_out);
+        tma_prefetch_desc(&g.tm_out);
     }
     if (warp == 1) tmem_alloc(&bars->tmem_base, kNAcc * kNBN);
     tc_fence_before();
@@ -275,19 +276,21 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
                         goto producer_done;
                     }
                     uint8_t *slotp = ring + r * g.slot_bytes;
-                    const uint32_t tx = nt * kNABytes + (st == 0 ? nvb * G::BOX_BYTES : 0);
+                    const int a_rows = cs.box[0] + (nt > 1 ? cs.box[1] : 0);
+                    const uint32_t tx = a_rows * 128 + (st == 0 ? nvb * G::BOX_BYTES : 0);
                     mbar_arrive_expect_tx(&bars->wfull[r], tx);
                     for (int t = 0; t < nt; ++t) {
                         // the unit's row tile t: weight rows m0 .. m0 + 127
                         const int m0 = (r0 + t) * 128;
                         const bool tail =
                             cs.tail_hi > cs.tail_lo && m0 < cs.tail_hi && m0 + 128 > cs.tail_lo;
-                        tma_load_2d(slotp + t * kNABytes, tail ? &cs.tm_wt : &cs.tm_w,
+                        const int map = t > 0 && cs.box[1] != cs.box[0];
+                        tma_load_2d(slotp + t * kNABytes, tail ? &cs.tm_wt : &cs.tm_w[map],
                                     &bars->wfull[r], kb * G::BK, tail ? m0 - cs.tail_row0 : m0);
                     }
                     if (st == 0)  // the first stage's activations, shared by the row tiles
                         for (int jb = 0; jb < nvb; ++jb)
-                            tma_load_2d(slotp + g.ra * kNABytes + jb * G::BOX_BYTES, &g.tm_b,
+                            tma_load_2d(slotp + g.b_off + jb * G::BOX_BYTES, &g.tm_b,
                                         &bars->wfull[r], n0 + jb * G::BOX_N, kb * G::BK);
                     pending |= 1u << r;
                     pending_ph = (pending_ph & ~(1u << r)) | (rph << r);
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
             // of operand buffer 0
             const uint64_t a_desc0 = smem_desc(smem_u32(ring), 16, 1024, SMEM_SW128);
             const uint64_t b_desc0 =
-                smem_desc(smem_u32(ring) + g.ra * kNABytes, G::BOX_BYTES, 1024, SMEM_SW128);
+                smem_desc(smem_u32(ring) + g.b_off, G::BOX_BYTES, 1024, SMEM_SW128);
             const uint64_t x_desc0 = smem_desc(smem_u32(xbuf), 16, 1024, SMEM_SW128);
             int slot, j, st, r0, nt;
             for (int u = 0; walk.next(slot, j, st, r0, nt); ++u) {
@@ -499,7 +502,7 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            tma_store_2d(&cs.tm_out, b0, nc, warp_row0);
+                            tma_store_2d(&g.tm_out, b0, nc, warp_row0);
                             bulk_commit();
                         }
                         continue;
@@ -516,10 +519,13 @@ __global__ void __launch_bounds__(n_threads(EW), 1) tc_narrow_kernel(const __gri
                                 *reinterpret_cast<uint32_t *>(xs + kmaj<2>(k0, lc + 16 * h + u)) =
                                     pack_bf16x2(v[2 * u], v[2 * u + 1]);
                         } else {
+                            // rows past M are zeros for the next stage (its weights there are
+                            // too, but this tile's were whatever lay behind its box)
+                            const uint32_t keep = row < cs.M ? 0xffffu : 0u;
 #pragma unroll
                             for (int u = 0; u < 32; ++u)
                                 *reinterpret_cast<uint16_t *>(xs + kmaj<2>(row, lc + u)) =
-                                    (uint16_t)(pack_bf16x2(v[u], v[u]) & 0xffffu);
+                                    (uint16_t)(pack_bf16x2(v[u], v[u]) & keep);
                         }
                     } else {
                         if (cs.permute && full && row < (cs.M / 4) * 4) {
@@ -589,6 +595,18 @@ namespace {
 // the reference's chain table: INT8 N = 65536 56 -> 48 us, BF16 44 -> 40 us),
 // four where a two-tile unit needs the ring's room (eight there cost a ring slot
 // and up to 16 %).
+// Weight rows loaded per row tile of a unit: what there is, in whole 8-row swizzle atoms.
+// The MMA reads 128 rows from a tile's start all the same; the rows behind a box are
+// other bytes of the slot (or what follows the ring), and their results are not used.
+// Full boxes of zero rows cost ring slots: two for M = 144 (BF16 16384 x 1296, 144, 32,
+// 192 25.7 -> 24.1 us).
+void narrow_boxes(int M, bool last, int (&box)[2])
+{
+    auto pad8 = [](int r) { return (std::min(r, 128) + 7) / 8 * 8; };
+    box[0] = pad8(M);
+    box[1] = !last && M > 128 ? pad8(M - 128) : 0;
+}
+
 template <int OP>
 bool narrow_layout(const StageArgs *st, int n, NarrowArgs &A)
 {
@@ -598,9 +616,15 @@ bool narrow_layout(const StageArgs *st, int n, NarrowArgs &A)
         ra = std::max(ra, (st[i].M + 127) / 128);
         xkb = std::max(xkb, (st[i].M + G::BK - 1) / G::BK);
     }
-    A.ra = ra;
     A.epi_warps = ra == 1 ? 8 : 4;
-    A.slot_bytes = ra * kNABytes + G::B_BYTES;
+    A.b_off = A.slot_bytes = 0;
+    for (int i = 0; i < n; ++i) {
+        int box[2];
+        narrow_boxes(st[i].M, i + 1 == n, box);
+        const int a_bytes = (box[0] + box[1]) * 128;
+        if (i == 0) A.b_off = a_bytes;
+        A.slot_bytes = std::max(A.slot_bytes, a_bytes + (i == 0 ? G::B_BYTES : 0));
+    }
     A.x_bytes = xkb * kNKbBytes;
     const int fixed = n_fixed(A.epi_warps);
     // at most two column blocks in flight (FG_NARROW_XSLOTS=<1..4> overrides):
@@ -673,11 +697,11 @@ cudaError_t narrow_attr(int smem)
     int dev = 0;
     cudaGetDevice(&dev);
     if (done[dev & 63] >= smem) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(tc_narrow_kernel<OP, 4>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kNMaxSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(tc_narrow_kernel<OP, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kNMaxSmem);
+    auto allow = [](auto *kernel) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kNMaxSmem);
+    };
+    cudaError_t e = allow(tc_narrow_kernel<OP, 4>);
+    if (e == cudaSuccess) e = allow(tc_narrow_kernel<OP, 8>);
     if (e != cudaSuccess) return e;
     done[dev & 63] = kNMaxSmem;
     return cudaSuccess;
@@ -725,12 +749,19 @@ cudaError_t plan_narrow_op(const StageArgs *st, int n, int num_sms, NarrowArgs &
         for (int i = 0; i < n; ++i) {
             const StageArgs &a = st[i];
             NarrowStage &cs = A.st[i];
-            if (!make_map(&cs.tm_w, dt, G::elt, a.w, a.M, a.K, a.ld_w, G::BK, 128))
-                return cudaErrorNotSupported;
-            cs.tm_wt = cs.tm_w;
+            narrow_boxes(a.M, i + 1 == n, cs.box);
+            for (int t = 0; t < 2; ++t) {
+                const int rows = cs.box[t] ? cs.box[t] : cs.box[0];
+                if (!make_map(&cs.tm_w[t], dt, G::elt, a.w, a.M, a.K, a.ld_w, G::BK, rows))
+                    return cudaErrorNotSupported;
+            }
+            cs.tm_wt = cs.tm_w[0];
+            // at most 8 rows, which no tile edge cuts: row 128 is not inside [12q, 12q + 8)
+            // for an M of whole fours, and other M end the block at 128
+            const int tail_box = i + 1 < n && a.tail_lo >= 128 ? cs.box[1] : cs.box[0];
             if (a.tail_hi > a.tail_lo &&
-                !make_map(&cs.tm_wt, dt, G::elt, a.w_tail, a.M - a.tail_row0, a.K, a.ld_w_tail,
-                          G::BK, 128))
+                !make_map(&cs.tm_wt, dt, G::elt, a.w_tail, a.M - a.tail_row0, a.K, a.ld_w_tail, G::BK,
+                          tail_box))
                 return cudaErrorNotSupported;
             cs.M = a.M;
             cs.K = a.K;
@@ -741,8 +772,7 @@ cudaError_t plan_narrow_op(const StageArgs *st, int n, int num_sms, NarrowArgs &
             cs.w_tail = static_cast<const uint8_t *>(a.w_tail);
             cs.ld_w_tail = a.ld_w_tail;
             cs.out_rows = a.m_written;
-            if (i + 1 == n && !make_out_map(&cs.tm_out, a)) return cudaErrorNotSupported;
-            if (i + 1 < n) cs.tm_out = cs.tm_w;
+            if (i + 1 == n && !make_out_map(&A.tm_out, a)) return cudaErrorNotSupported;
         }
         if (!narrow_layout<OP>(st, n, A)) return cudaErrorNotSupported;
         A.b = st[0].x;
