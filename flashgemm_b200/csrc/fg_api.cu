@@ -316,8 +316,8 @@ size_t chain_scratch(int dtype, int algo, long N, int n, const long *M, const lo
             size_t items = 0;
             for (int i = 0; i < n; ++i) items += (size_t)((M[i] + 255) / 256) * ((N + 255) / 256);
             s += carve_size(items * 2 * 10 * 8);
-            // or of the narrow kernel: one row per (column block, unit) at most
-            s += carve_size((size_t)((N + 127) / 128) * (n - 1 + (M[n - 1] + 127) / 128) *
+            // or of the narrow kernel: every CTA's rows for the most column blocks of one
+            s += carve_size((size_t)((N + 127) / 128) * 2 * (n - 1 + (M[n - 1] + 127) / 128) *
                             kNarrowTraceFields * 8);
         }
     }
@@ -394,7 +394,7 @@ int launch_stages(DevCtx *c, int kind, std::vector<StageArgs> &stages, long N)
         if (plan_narrow(stages.data(), n, c->sms, P, grid) == cudaSuccess) {
             double fl = 0.0;
             for (auto &st : stages) fl += gemm_flops(st.M, st.N, st.K);
-            // FG_TRACE_DIR=<dir>: a per-unit timeline of every narrow launch
+            // FG_TRACE_DIR=<dir>: a per-tile timeline of every narrow launch
             static const char *trace_dir = getenv("FG_TRACE_DIR");
             size_t trace_words = 0;
             P.trace = nullptr;
@@ -419,7 +419,7 @@ int launch_stages(DevCtx *c, int kind, std::vector<StageArgs> &stages, long N)
                                "mma_start,mma_end,epi_start,epi_end\n");
                     for (size_t r = 0; r < trace_words / kNarrowTraceFields; ++r) {
                         const unsigned long long *v = &h[r * kNarrowTraceFields];
-                        if (!v[1]) continue;  // a unit the CTA did not have
+                        if (!v[1]) continue;  // a tile the CTA did not have
                         fprintf(f, "%zu,%zu,%llu,%llu,%llu,%llu,%llu", r / P.trace_units,
                                 r % P.trace_units, v[0] & 0xff, (v[0] >> 8) & 0xffff,
                                 (v[0] >> 24) & 0xff, (v[0] >> 32) & 0xff, v[0] >> 40);

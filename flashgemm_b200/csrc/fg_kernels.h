@@ -206,47 +206,43 @@ cudaError_t launch_single_group(const GroupLaunch &g, const void *tables_dev, in
 // ------------------------------------------------------------------ narrow chains
 //
 // BF16 / INT8 chains whose intermediates have at most kNarrowRows rows keep
-// them on chip (fg_narrow.cu): one CTA per 128-column block, the first stage's
-// operands streamed through a TMA ring, each intermediate converted as the
-// reference does and written K-major into shared memory, only the last
-// stage's result stored. Any K_1, any last width.
+// them on chip (fg_narrow.cu): one CTA per 128-column block, the operands
+// streamed through a TMA ring, each intermediate converted as the reference
+// does and kept in tensor memory, only the last stage's result stored. Any
+// K_1, any last width.
 
 constexpr int kNarrowRows = 256;
 constexpr int kNarrowMaxStages = 8;
 constexpr int kNarrowMaxRing = 8;
-constexpr int kNarrowMaxX = 4;       // column blocks in flight per CTA, at most
 
-struct alignas(64) NarrowStage {
-    // weights, K-major boxes of 128-byte rows, of `box` rows for row tiles 0 and 1 of an
-    // intermediate (the last stage: 0 for all of its tiles)
-    CUtensorMap tm_w[2];
-    CUtensorMap tm_wt;   // INT8 reference tail block, for the one row tile that holds it
-    int box[2];
+struct NarrowStage {
     int M, K;
     int permute;         // the reference's panel permutation between stages
+    int rows, tiles;     // rows per tile (a multiple of 16); more than one tile: last stage only
     int tail_lo, tail_hi, tail_row0;
     const uint8_t *w_tail;
     long ld_w_tail;
-    int out_rows;        // last stage: rows stored (INT8 reference: 4 * floor(M / 4))
 };
 
 struct alignas(64) NarrowArgs {
+    CUtensorMap tm_w[kNarrowMaxStages];   // weights, K-major boxes of `rows` rows
+    CUtensorMap tm_wt[kNarrowMaxStages];  // INT8 reference tail block, for the tiles that hold tail rows
+    CUtensorMap tm_x;    // B (K_1 x N), MN-major boxes
     NarrowStage st[kNarrowMaxStages];
-    CUtensorMap tm_b;    // first stage's activations (K_1 x N), MN-major boxes
-    CUtensorMap tm_out;  // last stage: the result (staged TMA stores)
-    const void *b;       // the same, for the INT8 tail correction
+    const uint8_t *b;    // the same, for the INT8 tail correction
     long ldb;
+    uint32_t *out;       // C (FP32 or int32)
+    long ldo;
+    int out_rows;        // rows stored (INT8 reference: 4 * floor(M / 4))
     int n, N, nblocks;
     int op;              // OperandKind
-    // shared memory layout of the launch: ring slots of slot_bytes (a unit's weight
-    // boxes, then at b_off the first stage's activation boxes), xslots operand buffers
-    // of x_bytes (one per column block in flight, 1 to kNarrowMaxX), smem bytes in all
-    int ring, slot_bytes, b_off, x_bytes, xslots, smem;
-    int epi_warps;       // 4 or 8 epilogue warps
+    int ring, slot_bytes, smem;        // ring slots and their bytes, shared memory in all
+    int acc, acc_step, tmem_cols;      // TMEM columns: first of the accumulators, from one to the next, in all
+    int per_sm;          // CTAs per SM
     int *status;
-    // optional (else null): kNarrowTraceFields %globaltimer stamps per (CTA, unit)
+    // optional (else null): kNarrowTraceFields %globaltimer stamps per (CTA, tile)
     unsigned long long *trace;
-    int trace_units;     // units per CTA the trace holds
+    int trace_units;     // tiles per CTA the trace holds
 };
 constexpr int kNarrowTraceFields = 8;
 
@@ -257,7 +253,7 @@ bool narrow_preferred(const StageArgs *st, int n, int num_sms);
 // for the last few operand sets); cudaErrorNotSupported when it does not qualify.
 cudaError_t plan_narrow(const StageArgs *st, int n, int num_sms, NarrowArgs &out, int &grid);
 cudaError_t launch_narrow(NarrowArgs &P, int grid, int *status, cudaStream_t s);
-// Work units one CTA of a narrow launch walks at most (the trace's rows per CTA).
+// Tiles one CTA of a narrow launch walks at most (the trace's rows per CTA).
 int narrow_units_per_cta(const NarrowArgs &P, int grid);
 
 // ------------------------------------------------------------------ panel-resident chains
