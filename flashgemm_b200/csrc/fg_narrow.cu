@@ -110,21 +110,32 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
 
-    // k-block kb of a stage's tile t into ring slot i: the weights' box, and B's for stage 0
-    auto load = [&](const NarrowStage &cs, int st, int blk, int t, int kb, int i) {
-        const int m0 = t * cs.rows, n0 = blk * kNBN;
-        int nvb = 0;
-        if (st == 0) {  // boxes that start inside N
-            nvb = (g.N - n0 + G::BOX_N - 1) / G::BOX_N;
-            nvb = nvb < G::NBOX ? nvb : G::NBOX;
-        }
-        uint8_t *p = smem + i * g.slot_bytes;
-        mbar_arrive_expect_tx(&bars->full[i], (uint32_t)(cs.rows * 128 + nvb * G::BOX_BYTES));
+    // What a tile's k-blocks are loaded with: the weights' map and row, the boxes of B that
+    // start inside N (stage 0).
+    struct Tile {
+        const CUtensorMap *w;
+        uint32_t bytes;
+        int wy, nvb, n0;
+    };
+    auto tile_of = [&](const NarrowStage &cs, int st, int blk, int t) {
+        Tile q;
+        const int m0 = t * cs.rows;
         const bool tail = cs.tail_hi > cs.tail_lo && m0 < cs.tail_hi && m0 + cs.rows > cs.tail_lo;
-        for (int j = 0; j < nvb; ++j)
-            tma_load_2d(p + j * G::BOX_BYTES, &g.tm_x, &bars->full[i], n0 + j * G::BOX_N, kb * G::BK);
-        tma_load_2d(p + kNXBytes, tail ? &g.tm_wt[st] : &g.tm_w[st], &bars->full[i], kb * G::BK,
-                    tail ? m0 - cs.tail_row0 : m0);
+        q.n0 = blk * kNBN;
+        q.nvb = st == 0 ? min(G::NBOX, (g.N - q.n0 + G::BOX_N - 1) / G::BOX_N) : 0;
+        q.w = tail ? &g.tm_wt[st] : &g.tm_w[st];
+        q.wy = tail ? m0 - cs.tail_row0 : m0;
+        q.bytes = (uint32_t)(cs.rows * 128 + q.nvb * G::BOX_BYTES);
+        return q;
+    };
+    // k-block kb of a tile into ring slot i
+    auto load = [&](const Tile &q, int kb, int i) {
+        uint8_t *p = smem + i * g.slot_bytes;
+        mbar_arrive_expect_tx(&bars->full[i], q.bytes);
+        if (q.nvb > 0) tma_load_2d(p, &g.tm_x, &bars->full[i], q.n0, kb * G::BK);
+        if (G::NBOX > 1 && q.nvb > 1)
+            tma_load_2d(p + G::BOX_BYTES, &g.tm_x, &bars->full[i], q.n0 + G::BOX_N, kb * G::BK);
+        tma_load_2d(p + kNXBytes, q.w, &bars->full[i], kb * G::BK, q.wy);
     };
     const int first_loads = min(g.ring, (g.st[0].K + G::BK - 1) / G::BK);
 
@@ -143,7 +154,8 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
         fence_mbar_init();
         // the ring's first round needs no wait: under way before the CTA meets
         overlap_wait();
-        for (int kb = 0; kb < first_loads; ++kb) load(g.st[0], 0, blockIdx.x, 0, kb, kb);
+        const Tile q0 = tile_of(g.st[0], 0, blockIdx.x, 0);
+        for (int kb = 0; kb < first_loads; ++kb) load(q0, kb, kb);
         for (int i = 1; i < g.n; ++i) {
             tma_prefetch_desc(&g.tm_w[i]);
             if (g.st[i].tail_hi > g.st[i].tail_lo) tma_prefetch_desc(&g.tm_wt[i]);
@@ -176,15 +188,20 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
                                        (unsigned long long)t << 24 | 1ull << 32 | (unsigned long long)sm << 40);
                             ntrace(g, u, NT_PROD_START, globaltimer_ns());
                         }
+                        const Tile q = tile_of(cs, st, blk, t);
+                        bool ready = false;
                         for (int kb = 0; kb < nkb; ++kb) {
                             if (skip > 0) {  // loaded above
                                 --skip;
                             } else {
-                                if (!mbar_wait(&bars->empty[s], ph ^ 1, status, KERR_WAIT_EMPTY)) {
+                                if (!ready && !mbar_wait(&bars->empty[s], ph ^ 1, status, KERR_WAIT_EMPTY)) {
                                     n_set_abort(bars);
                                     goto producer_done;
                                 }
-                                load(cs, st, blk, t, kb, s);
+                                // the next slot, asked now and looked at after these loads are issued
+                                const int s1 = s + 1 == g.ring ? 0 : s + 1;
+                                ready = mbar_test(&bars->empty[s1], s1 ? ph ^ 1 : ph);
+                                load(q, kb, s);
                                 pending |= 1u << s;
                                 pending_ph = (pending_ph & ~(1u << s)) | (ph << s);
                             }
