@@ -15,9 +15,12 @@
 // 64-clock MMA, all that shared memory delivers, beside what TMA writes; here an MMA reads 4
 // KB of activations (later stages: none, A is in TMEM) and 32 bytes per real row.
 // Measured (B200, us a call, before -> now; before, the rows were the MMA's M and the
-// intermediates lay in shared memory): BF16 16384 x 1296, 144, 32, 192 24.1 -> 17.7, INT8
-// 4096 x 4800, 192, 56, 336 37.0 -> 25.8; 65536 x 288, 32, 24, 144 33 -> 22.5 (BF16), 30 ->
-// 17.8 (INT8); 20000 x 64, 128, 1024 33 -> 31 (BF16), 40 -> 31 (INT8).
+// intermediates lay in shared memory): BF16 16384 x 1296, 144, 32, 192 24.1 -> 17.2, INT8
+// 4096 x 4800, 192, 56, 336 37.0 -> 25.4; 65536 x 288, 32, 24, 144 33 -> 22.5 (BF16), 30 ->
+// 17.8 (INT8); 20000 x 64, 128, 1024 33 -> 31 (BF16), 40 -> 31 (INT8). What is left there:
+// the first stage's k-blocks come from L2 at 13 TB/s (BF16 table chain), or 32 blocks leave
+// 116 SMs idle (INT8; its k-blocks shared by a cluster of four CTAs, sums exchanged over
+// distributed shared memory, took 26.8 us: the exchange costs what the split saves).
 // Eight epilogue warps, not four: 65536 x 256, 256, 256 44.3 -> 39.4 (BF16), 43.2 -> 35.4 (INT8).
 //
 // INT8 reference tail rows (multigemm/src/kernel_int8.h:771-1057): their weights come
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
             uint32_t ph = 0, pending = (1u << first_loads) - 1, pending_ph = 0;
             for (int blk = blockIdx.x; blk < g.nblocks; blk += gridDim.x) {
                 for (int st = 0; st < g.n; ++st) {
-                    const NarrowStage &cs = bars->st[st];
+                    const NarrowStage cs = bars->st[st];  // in registers
                     const int nkb = (cs.K + G::BK - 1) / G::BK;
                     for (int t = 0; t < cs.tiles; ++t, ++u) {
                         if (g.trace) {
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
             bool ok = true;
             for (int blk = blockIdx.x; ok && blk < g.nblocks; blk += gridDim.x) {
                 for (int st = 0; ok && st < g.n; ++st) {
-                    const NarrowStage &cs = bars->st[st];
+                    const NarrowStage cs = bars->st[st];  // in registers
                     const int K = cs.K, ntiles = cs.tiles;
                     const int nkb = (K + G::BK - 1) / G::BK;
                     const uint32_t idesc = G::idesc(st == 0, cs.rows);
@@ -314,7 +317,7 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
             const int c0 = blk * kNBN + quarter * 32, col = c0 + lane;
             const bool panel = c0 + 32 <= g.N;  // a whole panel: permuted
             for (int st = 0; ok && st < g.n; ++st) {
-                const NarrowStage &cs = bars->st[st];
+                const NarrowStage cs = bars->st[st];  // in registers
                 const bool last = st + 1 == g.n;
                 const bool tails = OP == OP_I8 && cs.tail_hi > cs.tail_lo;
                 // INT8 tails: the first quad of this column's input; of B it is fetched while
