@@ -23,10 +23,13 @@
 // What bounds it: the thread that issues the MMAs (about 70 clocks for each, 67 for a
 // commit, 96 for a wait that is already over) and the tensor pipe (three TF32 products
 // per 8 k of 48 clocks each up to 96 rows, rows / 2 above), hence one MMA for two of the
-// products where it fits, one commit per k-block, and waits tested ahead; and, on many columns, reading B once. The launch-per-stage
-// path that it replaces wrote B's split to memory and read it back (3x its bytes)
-// and paid a launch and a memory round trip per stage. Measured (B200, us a call, that
-// path -> this): SPLICE_NUMBERS
+// products where it fits, one commit per k-block, and waits tested ahead; and, on many
+// columns, reading B once. The launch-per-stage path that it replaces wrote B's split to
+// memory and read it back (3x its bytes) and paid a launch and a memory round trip per
+// stage. Measured (B200, us a call, that
+// path -> this): 12544 x 864, 96, 24, 144 102 -> 33; 65536 x 288, 32, 24, 144 159 -> 53;
+// 50176 x 288, 32, 16, 96 121 -> 41; 16384 x 1296, 144, 32, 192 181 -> 64; 3136 x the same
+// 81 -> 60.
 //
 // The arithmetic is that path's: per 8 k the correction terms lo * hi, then hi * lo,
 // into their own accumulator and hi * hi into the chunk's (hi * [hi | lo] as one MMA over the
