@@ -15,8 +15,8 @@
 // 64-clock MMA, all that shared memory delivers, beside what TMA writes; here an MMA reads 4
 // KB of activations (later stages: none, A is in TMEM) and 32 bytes per real row.
 // Measured (B200, us a call, before -> now; before, the rows were the MMA's M and the
-// intermediates lay in shared memory): BF16 16384 x 1296, 144, 32, 192 24.1 -> 17.2, INT8
-// 4096 x 4800, 192, 56, 336 37.0 -> 25.4; 65536 x 288, 32, 24, 144 33 -> 22.5 (BF16), 30 ->
+// intermediates lay in shared memory): BF16 16384 x 1296, 144, 32, 192 24.1 -> 16.9, INT8
+// 4096 x 4800, 192, 56, 336 37.0 -> 25.3; 65536 x 288, 32, 24, 144 33 -> 22.5 (BF16), 30 ->
 // 17.8 (INT8); 20000 x 64, 128, 1024 33 -> 31 (BF16), 40 -> 31 (INT8). What is left there:
 // the first stage's k-blocks come from L2 at 13 TB/s (BF16 table chain), or 32 blocks leave
 // 116 SMs idle (INT8; its k-blocks shared by a cluster of four CTAs, sums exchanged over
@@ -244,9 +244,10 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
                         ++xr;
                     }
                     for (int t = 0; ok && t < ntiles; ++t, ++tiles) {
-                        // accumulator tiles & 1; the tile before is read first where this is a new
-                        // stage (its accumulators may overlie), else only the one before that
-                        if (t == 0 && tiles > 0)
+                        // accumulator t & 1; the tile before is read first where this is a new stage
+                        // (its accumulators may overlie; past the first, xready came after that
+                        // read), else only the one before that
+                        if (t == 0 && st == 0 && tiles > 0)
                             ok = mbar_wait(&bars->dempty[(tiles - 1) & 1u], ((tiles - 1) >> 1) & 1u, status,
                                            KERR_WAIT_ACC_EMPTY);
                         else if (t > 1)
@@ -283,9 +284,18 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
                                     }
                                 }
                             } else {
-                                for (int k = 0; k < steps; ++k) {
-                                    tc_mma_ts<KIND>(d_tmem, tmem_base + (kb * 4 + k) * 8, w + k * 2, idesc, more);
-                                    more = 1;
+                                const uint32_t a = tmem_base + kb * 32;
+                                if (steps == 4) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k) {
+                                        tc_mma_ts<KIND>(d_tmem, a + k * 8, w + k * 2, idesc, more);
+                                        more = 1;
+                                    }
+                                } else {
+                                    for (int k = 0; k < steps; ++k) {
+                                        tc_mma_ts<KIND>(d_tmem, a + k * 8, w + k * 2, idesc, more);
+                                        more = 1;
+                                    }
                                 }
                             }
                             tc_commit(&bars->empty[s]);
