@@ -16,7 +16,7 @@
 // KB of activations (later stages: none, A is in TMEM) and 32 bytes per real row.
 // Measured (B200, us a call, before -> now; before, the rows were the MMA's M and the
 // intermediates lay in shared memory): BF16 16384 x 1296, 144, 32, 192 24.1 -> 16.9, INT8
-// 4096 x 4800, 192, 56, 336 37.0 -> 25.3; 65536 x 288, 32, 24, 144 33 -> 22.5 (BF16), 30 ->
+// 4096 x 4800, 192, 56, 336 37.0 -> 24.9; 65536 x 288, 32, 24, 144 33 -> 22.5 (BF16), 30 ->
 // 17.8 (INT8); 20000 x 64, 128, 1024 33 -> 31 (BF16), 40 -> 31 (INT8). What is left there:
 // the first stage's k-blocks come from L2 at 13 TB/s (BF16 table chain), or 32 blocks leave
 // 116 SMs idle (INT8; its k-blocks shared by a cluster of four CTAs, sums exchanged over
@@ -359,13 +359,17 @@ __global__ void __launch_bounds__(kNThreads, 2) tc_narrow_kernel(const __grid_co
                     auto rows16 = [&](uint32_t (&v)[16], int c) {
                         const int r0 = m0 + c * 16;
                         if (tails && r0 < cs.tail_hi && r0 + 16 > cs.tail_lo) {
+// tail_lo and tail_hi are whole quads of rows: warp-uniform tests per quad
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (r0 + j >= cs.tail_lo && r0 + j < cs.tail_hi) {  // warp-uniform
-                                    const uint32_t w = __shfl_sync(0xffffffffu, wq, r0 + j - cs.tail_lo);
-                                    int r;
-                                    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(xq), "r"((int)v[j]));
-                                    v[j] = (uint32_t)r;
+                            for (int q = 0; q < 16; q += 4)
+                                if (r0 + q >= cs.tail_lo && r0 + q < cs.tail_hi) {
+#pragma unroll
+                                    for (int j = q; j < q + 4; ++j) {
+                                        const uint32_t w = __shfl_sync(0xffffffffu, wq, r0 + j - cs.tail_lo);
+                                        int r;
+                                        asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(xq), "r"((int)v[j]));
+                                        v[j] = (uint32_t)r;
+                                    }
                                 }
                         }
                         if (last) {
