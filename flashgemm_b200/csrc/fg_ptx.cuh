@@ -468,12 +468,6 @@ __device__ __forceinline__ void tmem_st_32x32b_x4(uint32_t taddr, const uint32_t
                  "r"(r[2]), "r"(r[3]), "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ uint32_t tmem_ld_32x32b_x1(uint32_t taddr)
-{
-    uint32_t r;
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr));
-    return r;
-}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
