@@ -128,7 +128,7 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
 #pragma unroll
     for (int q = 0; q < B_P; ++q) {
         const int c = (b_c + q * NT) * EB, gn = n0 + c;
-        b_bytes[q] = min(max((N - gn) * 4, 0), 4 * EB);
+        b_bytes[q] = 4 * min(max(N - gn, 0), EB);  // clamped first: 4 N may not fit in an int
         b_src[q] = p.B + (b_bytes[q] ? gn : 0) + (long)b_r * p.ldb;
         b_dst[q] = sbase + (BM * BK + b_r * BN + c) * 4;
     }
@@ -160,7 +160,7 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
                 const int r = a_r + v * A_R;
                 if (BM % A_R && r >= BM) break;
                 const int gk = k0 + a_c * EA;
-                const int n = min(max((K - gk) * 4, 0), 4 * EA);
+                const int n = 4 * min(max(K - gk, 0), EA);
                 copy_async<EA>(a_dst(r) + off, p.A + (long)min(m0 + r, M - 1) * p.lda + (n ? gk : 0), n);
             }
 #pragma unroll

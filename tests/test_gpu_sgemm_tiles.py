@@ -48,3 +48,21 @@ def test_sgemm_tiles_bitexact(shape, offsets):
     fg.sgemm_dev(c, a, b, M, N, K)
     torch.cuda.synchronize()
     np.testing.assert_array_equal(c.cpu().numpy()[rows], want)
+
+
+@pytest.mark.parametrize("N", [(1 << 29) + 100, (1 << 29) + 101, 1 << 30],
+                         ids=["2^29+100", "2^29+101", "2^30"])
+def test_more_columns_than_a_31_bit_byte_count(N):
+    """Rows of 2 GB and more, with and without 16-byte-aligned rows: every column is
+    computed. Small whole numbers, so that every sum is exact."""
+    import torch
+    import flashgemm_b200 as fg
+    M, K = 2, 2
+    g = torch.Generator(device="cuda").manual_seed(N)
+    a = torch.tensor([[3.0, -2.0], [5.0, 7.0]], device="cuda")
+    b = torch.randint(-8, 9, (K, N), generator=g, device="cuda", dtype=torch.int8).float()
+    c = torch.full((M, N), 0.5, device="cuda")
+    fg.sgemm_dev(c, a, b, M, N, K)
+    torch.cuda.synchronize()
+    for i in range(M):
+        assert torch.equal(c[i], a[i, 0] * b[0] + a[i, 1] * b[1])
