@@ -209,12 +209,35 @@ int arena_reserve(DevCtx *c, size_t bytes)
     c->arena_cap = 0;
     size_t cap = bytes + bytes / 4 + (64u << 20);
     cudaError_t e = cudaMalloc(&c->arena, cap);
+    if (e != cudaSuccess && c->part) {  // calls need the arena, and do without K-block sums
+        cudaGetLastError();
+        cudaFree(c->part);
+        c->part = nullptr;
+        c->part_cap = 0;
+        e = cudaMalloc(&c->arena, cap);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(FG_ERR_NOMEM, "device scratch of %zu bytes: %s", cap, cudaGetErrorString(e));
     }
     c->arena_cap = cap;
     return FG_OK;
+}
+
+float *part_reserve(DevCtx *c, size_t bytes)
+{
+    if (bytes <= c->part_cap) return (float *)c->part;
+    if (c->part) {
+        if (cudaStreamSynchronize(c->work) != cudaSuccess) return nullptr;
+        cudaFree(c->part);
+    }
+    const size_t cap = bytes + bytes / 4 + (16u << 20);
+    c->part_cap = cudaMalloc(&c->part, cap) == cudaSuccess ? cap : 0;
+    if (!c->part_cap) {
+        cudaGetLastError();
+        c->part = nullptr;
+    }
+    return (float *)c->part;
 }
 
 // Table block of grouped launches (grow-only, like the arena).
@@ -1203,30 +1226,32 @@ int chain_va(int dtype, void *C, const void *B, long N, int num_gemm, va_list ap
 // (singlegemm/src/NN_mp.h:13, :247)
 constexpr int kSgemmKBlock = 2048;
 
-// Workspace of an FFMA SGEMM on stream s. A stream that is being captured gets none:
-// the graph would keep a pointer into the arena, which a later call may grow.
-size_t sgemm_workspace(DevCtx *c, long M, long N, long K, cudaStream_t s)
+// Workspace of an FFMA SGEMM on the work stream, in which its K blocks run side by side;
+// null where that does not pay or the memory cannot be had: they run in turn then, with the
+// same bits. Not in the arena, so that no call fails, and none loses its scratch, for it. A
+// stream that is being captured gets none: the graph would keep a pointer into a block that
+// a later call may grow.
+float *sgemm_workspace(DevCtx *c, long M, long N, long K)
 {
     const size_t bytes = ffma_sgemm_workspace(M, N, K, kSgemmKBlock, c->sms);
-    if (!bytes) return 0;
+    if (!bytes) return nullptr;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+    if (cudaStreamIsCapturing(c->work, &cap) != cudaSuccess) {
         cudaGetLastError();
-        return 0;
+        return nullptr;
     }
-    return cap == cudaStreamCaptureStatusNone ? carve_size(bytes) : 0;
+    return cap == cudaStreamCaptureStatusNone ? part_reserve(c, bytes) : nullptr;
 }
 
-// workspace: sgemm_workspace bytes of the arena are reserved for this call
 int run_sgemm(DevCtx *c, int algo, float *C, long ldc, const float *A, long lda, const float *B,
-              long ldb, long M, long N, long K, size_t workspace)
+              long ldb, long M, long N, long K)
 {
     if (algo == FG_F32_FFMA) {
         FfmaArgs f;
         f.M = (int)M; f.N = (int)N; f.K = (int)K;
         f.A = A; f.lda = lda; f.B = B; f.ldb = ldb; f.C = C; f.ldc = ldc;
         f.kblock = kSgemmKBlock;
-        f.part = workspace ? (float *)arena_take(c, workspace) : nullptr;
+        f.part = sgemm_workspace(c, M, N, K);
         f.ld_part = round_up(N, 4);
         return run_kernel(c, FG_PK_FFMA, gemm_flops(M, N, K), "ffma sgemm",
                           [&] { return launch_ffma_sgemm(f, c->sms, c->work); });
@@ -1249,12 +1274,9 @@ int host_sgemm(float *C, const float *A, const float *B, long M, long N, long K)
     const long ldk = round_up(K > 0 ? K : 1, 4), ldn = round_up(N, 4);
     size_t need = carve_size((size_t)M * ldk * 4) + carve_size((size_t)K * ldn * 4) +
                   carve_size((size_t)M * ldn * 4) + 4096;
-    size_t workspace = 0;
     if (algo == FG_F32_3XTF32) {
         long Ms[1] = {M}, Ks[1] = {K};
         need += chain_scratch(FG_DT_F32, algo, N, 1, Ms, Ks);
-    } else {
-        need += workspace = sgemm_workspace(c, M, N, K, c->stream);
     }
     if ((st = enter_stream(c, c->stream))) return st;
     if ((st = arena_reserve(c, need))) return st;
@@ -1265,7 +1287,7 @@ int host_sgemm(float *C, const float *A, const float *B, long M, long N, long K)
         CUDA_TRY(copy_rows(ad, ldk * 4, A, K * 4, K * 4, M, cudaMemcpyHostToDevice, c->stream));
         CUDA_TRY(copy_rows(bd, ldn * 4, B, N * 4, N * 4, K, cudaMemcpyHostToDevice, c->stream));
     }
-    if ((st = run_sgemm(c, algo, cd, ldn, ad, ldk, bd, ldn, M, N, K, workspace))) return st;
+    if ((st = run_sgemm(c, algo, cd, ldn, ad, ldk, bd, ldn, M, N, K))) return st;
     CUDA_TRY(copy_rows(C, N * 4, cd, ldn * 4, N * 4, M, cudaMemcpyDeviceToHost, c->stream));
     if ((st = collect_status(c))) return st;
     return ok();
@@ -1599,16 +1621,14 @@ FG_EXPORT int fg_sgemm_dev(float *C, const float *A, const float *B, long M, lon
     int st;
     if ((st = get_ctx(&c))) return st;
     std::lock_guard<std::mutex> lk(c->mu);
-    size_t need = 4096, workspace = 0;
+    size_t need = 4096;
     if (algo == FG_F32_3XTF32) {
         long Ms[1] = {M}, Ks[1] = {K};
         need += chain_scratch(FG_DT_F32, algo, N, 1, Ms, Ks);
-    } else {
-        need += workspace = sgemm_workspace(c, M, N, K, user_stream(stream));
     }
     if ((st = enter_stream(c, user_stream(stream)))) return st;
     if ((st = arena_reserve(c, need))) return st;
-    if ((st = run_sgemm(c, algo, C, N, A, K, B, N, M, N, K, workspace))) return st;
+    if ((st = run_sgemm(c, algo, C, N, A, K, B, N, M, N, K))) return st;
     return ok();
 }
 

@@ -116,6 +116,8 @@ struct DevCtx {
     char *arena = nullptr;
     size_t arena_cap = 0;
     size_t arena_off = 0;
+    char *part = nullptr;    // plain FP32 SGEMM: sums of K blocks that run side by side
+    size_t part_cap = 0;
     char *tab = nullptr;     // grouped launches: device copies of their tables
     size_t tab_cap = 0;
     int *status = nullptr;       // device word the kernels report into
@@ -141,6 +143,9 @@ int get_ctx(DevCtx **out);
 int arena_reserve(DevCtx *c, size_t bytes);
 int tab_reserve(DevCtx *c, size_t bytes);
 void *arena_take(DevCtx *c, size_t bytes);
+// Block of K-block sums (grow-only, given back when the arena cannot grow otherwise);
+// null where it cannot be had.
+float *part_reserve(DevCtx *c, size_t bytes);
 inline size_t carve_size(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 
 // Sequential 256-byte-aligned carving of a caller-owned device block.

@@ -2,6 +2,9 @@
 in M, N and K, K blocks of 2048 with remainders, rows and pointers that are not
 16-byte aligned, on device memory. Bit for bit the oracle's result (one FMA per k
 in increasing k, K cut into blocks of 2048), NaN and infinity included."""
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -66,3 +69,36 @@ def test_more_columns_than_a_31_bit_byte_count(N):
     torch.cuda.synchronize()
     for i in range(M):
         assert torch.equal(c[i], a[i, 0] * b[0] + a[i, 1] * b[1])
+
+
+NO_ROOM = """
+import torch
+import flashgemm_b200 as fg
+M = N = 512
+K = 800 * 2048                       # 838 MB of K-block sums
+g = torch.Generator(device="cuda").manual_seed(5)
+a = torch.rand(M, K, generator=g, device="cuda") - 0.5
+b = torch.rand(K, N, generator=g, device="cuda") - 0.5
+c = torch.zeros(M, N, device="cuda")
+fg.sgemm_dev(c, a, b, M, N, 32)      # the kernels are loaded, and what every call needs is there
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+filler = torch.empty(torch.cuda.mem_get_info()[0] - (400 << 20), dtype=torch.uint8, device="cuda")
+fg.sgemm_dev(c, a, b, M, N, K)
+torch.cuda.synchronize()
+in_turn = c.clone()
+del filler
+torch.cuda.empty_cache()
+c.zero_()
+fg.sgemm_dev(c, a, b, M, N, K)
+torch.cuda.synchronize()
+assert torch.equal(c, in_turn) and bool(c.any())
+print("SAME BITS")
+"""
+
+
+def test_no_room_for_k_block_sums():
+    """On a device too full for the sums of K blocks side by side the call runs them in turn,
+    with the same bits. In a process of its own, which has no workspace from earlier calls."""
+    out = subprocess.run([sys.executable, "-c", NO_ROOM], capture_output=True, text=True, timeout=300)
+    assert "SAME BITS" in out.stdout, out.stderr[-2000:]
