@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "fg_host.h"
+#include "fg_serve_rule.h"
 
 using namespace fg;
 using namespace fg::host;
@@ -41,6 +42,8 @@ struct fg_server_s {
         size_t bytes = 0;
         void *mem = nullptr;
         void *tab[3] = {nullptr, nullptr, nullptr};  // grouped tables per dtype
+        bool waits = false;   // a grid of it is a waiting one (fg_serve_rule.h)
+        bool spread = false;  // its grids run side by side
         int status = FG_OK;
     };
 
@@ -120,14 +123,21 @@ void server_finish(fg_server_s *s, fg_server_s::Batch *b, double t)
     s->free_slots.push_back(b->slot);
 }
 
+// What is in flight when a batch is launched.
+struct Beside {
+    bool alone = true;               // nothing
+    bool waiting = false;            // a batch with a waiting grid (fg_serve_rule.h)
+    std::vector<cudaEvent_t> spread; // ends of the batches whose grids run side by side
+};
+
 // Launches one batch: device copies of host operands on its slot's stream, one grouped
-// launch per dtype present, each as soon as the host has built it and on a stream of its
-// own (one dtype's last tiles leave SMs that the next one's first take), copies of host
-// results, an event. alone: no other batch is in flight, so that kernels whose CTAs wait
-// on no CTA still to be started may take every SM; others keep to the batch's cap.
+// launch per dtype present, each as soon as the host has built it, copies of host results,
+// an event. Where batch_mode allows it the dtypes' launches run side by side, each on a
+// stream of its own (one dtype's last tiles leave SMs that the next one's first take), and
+// on every SM when no other batch is in flight; others run in turn and keep to the batch's cap.
 // Measured (B200, burst of 48 mixed requests): all built, then launched in turn on half the
 // SMs each 1192 us, so 1040; with placing per tile before that 2280.
-int server_launch(fg_server_s *s, fg_server_s::Batch *b, bool alone)
+int server_launch(fg_server_s *s, fg_server_s::Batch *b, const Beside &beside)
 {
     DevCtx *c = s->c;
     const int slot = b->slot;
@@ -162,6 +172,7 @@ int server_launch(fg_server_s *s, fg_server_s::Batch *b, bool alone)
         int dtype;
         std::vector<fg_chain_desc> chains;
         double flops = 0.0;
+        int algo = 0, kernel = 0, order = 0;
     };
     Part per[3];
     per[0].dtype = FG_DT_BF16;
@@ -176,17 +187,27 @@ int server_launch(fg_server_s *s, fg_server_s::Batch *b, bool alone)
             }
     }
     std::stable_sort(per, per + 3, [](const Part &x, const Part &y) { return x.flops > y.flops; });
+    for (Part &p : per) {
+        if (p.chains.empty()) continue;
+        p.algo = p.dtype == FG_DT_F32 ? algo : 0;
+        p.kernel = g_group_kernel.load();
+        p.order = g_group_order.load();
+        group_resolve(c, p.dtype, p.algo, (int)p.chains.size(), p.chains.data(), p.kernel, p.order);
+        // the plain FP32 path has neither
+        if (!(p.dtype == FG_DT_F32 && algo == FG_F32_FFMA) && (p.kernel == GK_PAIR || !group_dynamic()))
+            b->waits = true;
+    }
+    const BatchMode mode = batch_mode(b->waits, beside.waiting, beside.alone, s->cap_given);
+    b->spread = mode.spread;
+    if (mode.after_spread)
+        for (cudaEvent_t ev : beside.spread) CUDA_TRY(cudaStreamWaitEvent(st, ev, 0));
     b->gx.resize(3);
     int launched = 0;
     for (int d = 0; d < 3; ++d) {
         if (per[d].chains.empty()) continue;
-        const int dtype = per[d].dtype, n = (int)per[d].chains.size();
-        const int a = dtype == FG_DT_F32 ? algo : 0;
-        int kernel = g_group_kernel.load(), order = g_group_order.load();
-        group_resolve(c, dtype, a, n, per[d].chains.data(), kernel, order);
-        const bool all_sms = alone && !s->cap_given && kernel != GK_PAIR && group_dynamic();
-        int e = group_build(c, dtype, a, kernel, order, n, per[d].chains.data(), cv, b->gx[d], status,
-                            all_sms ? c->sms : s->o.ctas_per_batch);
+        int e = group_build(c, per[d].dtype, per[d].algo, per[d].kernel, per[d].order,
+                            (int)per[d].chains.size(), per[d].chains.data(), cv, b->gx[d], status,
+                            mode.all_sms ? c->sms : s->o.ctas_per_batch);
         if (e) return e;
         if (cv.off > b->bytes) return fail(FG_ERR_NOMEM, "serving: admission estimate too small");
         CUDA_TRY(cudaMallocFromPoolAsync(&b->tab[d], group_tab_bytes(b->gx[d]), s->pool, st));
@@ -194,7 +215,7 @@ int server_launch(fg_server_s *s, fg_server_s::Batch *b, bool alone)
         ct.base = (char *)b->tab[d];
         group_place(b->gx[d], ct);
         cudaStream_t on = st;
-        if (launched > 0) {
+        if (mode.spread && launched > 0) {
             on = s->sides[2 * slot + launched - 1];
             cudaEvent_t ev = s->forks[2 * slot + launched - 1];
             CUDA_TRY(cudaEventRecord(ev, st));  // operands and tables are there
@@ -204,7 +225,7 @@ int server_launch(fg_server_s *s, fg_server_s::Batch *b, bool alone)
         if ((e = group_upload(b->gx[d], on, false))) return e;
         if ((e = group_launch(c, b->gx[d], on, false, status))) return e;
     }
-    for (int i = 1; i < launched; ++i) {  // the slot's stream goes on after all of them
+    for (int i = 1; mode.spread && i < launched; ++i) {  // the slot's stream goes on after all of them
         cudaEvent_t ev = s->forks[2 * slot + i - 1];
         CUDA_TRY(cudaEventRecord(ev, s->sides[2 * slot + i - 1]));
         CUDA_TRY(cudaStreamWaitEvent(st, ev, 0));
@@ -296,12 +317,17 @@ void server_dispatch_loop(fg_server_s *s)
         s->peak = std::max(s->peak, s->used);
         ++s->batches;
         s->batched += (long long)b->reqs.size();
-        const bool alone = s->inflight.empty();
+        Beside beside;
+        for (const fg_server_s::Batch *f : s->inflight) {
+            beside.alone = false;
+            beside.waiting = beside.waiting || f->waits;
+            if (f->spread) beside.spread.push_back(s->events[f->slot]);
+        }
         lk.unlock();
         int st;
         {
             std::lock_guard<std::mutex> g(s->c->mu);
-            st = server_launch(s, b, alone);
+            st = server_launch(s, b, beside);
         }
         if (st) {  // nothing more runs for this batch: return its memory to the pool
             cudaGetLastError();

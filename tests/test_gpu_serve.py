@@ -227,3 +227,41 @@ def test_load_shedding_bounds_queueing(fg):
     _oracle_check(fg, dt, As, B, want, N, Ms)
     srv.close()
     _release(sets)
+
+
+def test_mixed_dtypes_on_pair_kernels(fg):
+    """Batches of BF16, INT8 and FP32 (the most work) on two slots with the pair kernel, whose
+    CTAs wait on one another, between batches with the automatic choice: every request
+    completes, with the result it has alone."""
+    import torch
+    specs = [("f32", 512, [520, 640, 520]), ("bf16", 512, [264, 520, 200]), ("int8", 512, [264, 520, 200])]
+    sets = []
+    for j, (dt, K1, Ms) in enumerate(specs):
+        _, As, _ = oracle.chain_inputs(dt, 64, K1, Ms, seed=60 + j)
+        sets.append((dt, K1, Ms, [fg.Weights(dt, a) for a in As]))
+    N = 640
+    Bs = [_inputs(dt, K1, N, 6000 + j) for j, (dt, K1, _, _) in enumerate(sets)]
+    want = [_alone(fg, dt, W, B, N, Ms[-1]) for (dt, _, Ms, W), B in zip(sets, Bs)]
+    tB = [torch.from_numpy(B.view(np.int16) if B.dtype == np.uint16 else B).cuda() for B in Bs]
+    srv = fg.Server(max_batch=9, slots=2, max_wait_us=200)
+    try:
+        reqs = []
+        for burst in range(12):
+            fg.set_group_config(0 if burst % 3 else -1, -1)
+            for i in range(9):
+                j = i % 3
+                dt, _, Ms, W = sets[j]
+                C = torch.full((Ms[-1], N), 9, dtype=torch.int32 if dt == "int8" else torch.float32,
+                               device="cuda")
+                torch.cuda.current_stream().synchronize()
+                reqs.append((srv.submit(dt, W, tB[j], C), j, C))
+        for rid, _, _ in reqs:
+            srv.wait(rid)
+        st = srv.stats()
+    finally:
+        fg.set_group_config(-1, -1)
+        srv.close()
+    assert st["completed"] == len(reqs) and st["failed"] == 0
+    for _, j, C in reqs:
+        _same(sets[j][0], C.cpu().numpy(), want[j], sets[j][2][-1])
+    _release(sets)
