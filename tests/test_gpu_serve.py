@@ -265,3 +265,53 @@ def test_mixed_dtypes_on_pair_kernels(fg):
     for _, j, C in reqs:
         _same(sets[j][0], C.cpu().numpy(), want[j], sets[j][2][-1])
     _release(sets)
+
+
+def test_dtypes_of_a_batch_overlap(fg):
+    """Two requests of one batch, of different dtypes, each a chain of two tiles with a long
+    sum (two SMs): together they take about as long as the longer one."""
+    import torch
+    deep = {}
+    for dt, K in (("f32", 65536), ("bf16", 262144)):
+        tdt = torch.float32 if dt == "f32" else torch.bfloat16
+        Ms = [128, 128]
+        As = [torch.randn(m, k, device="cuda").div_(k ** 0.5).to(tdt) for m, k in zip(Ms, [K, 128])]
+        abi = [a if dt == "f32" else a.view(torch.int16) for a in As]
+        B = torch.randn(K, 64, device="cuda").to(tdt)
+        deep[dt] = ([fg.Weights(dt, a) for a in abi], B if dt == "f32" else B.view(torch.int16),
+                    torch.zeros(Ms[-1], 64, device="cuda"), torch.zeros(Ms[-1], 64, device="cuda"))
+    torch.cuda.synchronize()
+    srv = fg.Server(max_batch=8, slots=1)
+    fg.set_group_config(2, 0)  # 128 x 128 tiles, all stages in one launch
+
+    def passes(dts):
+        """Shortest time from a first request, alone in its batch, to the end of a second
+        batch with these dtypes."""
+        best = None
+        for _ in range(12):
+            srv.reset_stats()
+            W, B, C, _ = deep["f32"]
+            t0 = time.perf_counter()
+            ids = [srv.submit("f32", W, B, C)]
+            while srv.stats()["batches"] < 1 and time.perf_counter() - t0 < 1.0:
+                pass
+            ids += [srv.submit(dt, deep[dt][0], deep[dt][1], deep[dt][3]) for dt in dts]
+            for rid in ids:
+                srv.wait(rid)
+            t = time.perf_counter() - t0
+            if srv.stats()["batches"] == (2 if dts else 1):
+                best = t if best is None else min(best, t)
+        assert best is not None
+        return best
+
+    try:
+        alone = passes([])
+        one, two, both = (passes(d) - alone for d in (["f32"], ["bf16"], ["f32", "bf16"]))
+    finally:
+        fg.set_group_config(-1, -1)
+        srv.close()
+        for W, _, _, _ in deep.values():
+            for w in W:
+                w.release()
+    print(f"f32 {one * 1e6:.0f} us, bf16 {two * 1e6:.0f} us, both {both * 1e6:.0f} us")
+    assert both < max(one, two) + 0.5 * min(one, two), (one, two, both)
