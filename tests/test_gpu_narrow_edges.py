@@ -3,6 +3,10 @@ groups and the two row tiles of the last stage, columns around the
 32-column panels and the 128-column blocks, more blocks than SMs (two CTAs per SM), and
 infinities and NaN in one column, which must not reach another. The per-GEMM path computes
 the same products in the same order: the results are equal bit for bit."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -84,3 +88,34 @@ def test_one_bad_column_stays_alone(fg, value):
         fg.set_semantics("ref")
     assert np.array_equal(C, ref, equal_nan=True)
     assert np.isfinite(np.delete(C, 40, axis=1)).all() and not np.isfinite(C[:, 40]).any()
+
+
+TRACED = """
+import glob, os, sys
+sys.path.insert(0, sys.argv[1])
+import conftest, oracle
+import flashgemm_b200 as fg
+import test_gpu_narrow_edges as t
+fg.set_chain_mode("fused")
+fg.set_narrow("always")
+traces = lambda kind: len(glob.glob(os.path.join(os.environ["FG_TRACE_DIR"], kind + "_trace_*.csv")))
+for N, K1, Ms in t.SHAPES:
+    for dt in ("bf16", "int8"):
+        B, As, Ks = oracle.chain_inputs(dt, N, K1, Ms, seed=1)
+        for sem in ("ref", "math"):
+            fg.set_semantics(sem)
+            before = traces("narrow")
+            t._both(fg, dt, B, As, N, Ms, Ks)
+            assert traces("narrow") > before, (dt, sem, N, K1, Ms)
+assert traces("chain") == 0
+print("ALL NARROW")
+"""
+
+
+def test_edges_run_on_the_narrow_kernel(tmp_path):
+    """Every shape above, in both types and semantics, leaves the narrow kernel's timeline
+    and none of the fused kernel's."""
+    env = dict(os.environ, FG_TRACE_DIR=str(tmp_path))
+    out = subprocess.run([sys.executable, "-c", TRACED, os.path.dirname(os.path.abspath(__file__))],
+                         capture_output=True, text=True, timeout=300, env=env)
+    assert "ALL NARROW" in out.stdout, out.stderr[-2000:]
