@@ -73,3 +73,69 @@ def test_column_chain_unregistered_weights_and_odd_columns(N):
             fg.set_chain_mode("fused")
         out.append(c.cpu().numpy())
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("N", [1001, 5120])
+def test_column_chain_unregistered_weights_is_two_launches(N):
+    """The weights' split and the chain, where one launch per stage takes four."""
+    import torch
+    import flashgemm_b200 as fg
+    Ms = [96, 24, 144]
+    B, As, Ks = oracle.chain_inputs("f32", N, 866, Ms, seed=N)
+    b, a = torch.from_numpy(B).cuda(), [torch.from_numpy(x).cuda() for x in As]
+    c = torch.zeros(Ms[-1], N, device="cuda")
+    fg.set_f32_algo("3xtf32")
+    counts = []
+    for mode in ("fused", "per_gemm"):
+        fg.set_chain_mode(mode)
+        try:
+            before = fg.kernel_launches()
+            fg.chain_dev("f32", c, b, N, a, Ms, Ks)
+            fg.sync()
+            counts.append(fg.kernel_launches() - before)
+        finally:
+            fg.set_chain_mode("fused")
+    assert counts == [2, 4]
+
+
+@pytest.mark.parametrize("shape", [(300, 98, (16, 18, 17)), (300, 514, (144, 32, 192)), (300, 98, (50, 32, 400))],
+                         ids=["half-sm", "16-deep", "tiles"])
+def test_bad_values_as_per_stage(shape):
+    """Infinities, NaN and sums past the largest FP32 in B and in the weights: the same bits,
+    or NaN, as one launch per stage, and every other column stays finite."""
+    import torch
+    import flashgemm_b200 as fg
+    N, K1, Ms = shape
+    Ms = list(Ms)
+    B, As, Ks = oracle.chain_inputs("f32", N, K1, Ms, seed=K1)
+    B, As = np.array(B), [np.array(a) for a in As]
+    B[5, 40], B[K1 - 1, 131], B[7, 250] = np.inf, np.nan, 3.4e38
+    fg.set_f32_algo("3xtf32")
+    b = torch.from_numpy(B).cuda()
+
+    def run(weights):
+        out = []
+        W = [fg.Weights("f32", a) for a in weights]
+        for mode in ("fused", "per_gemm"):
+            fg.set_chain_mode(mode)
+            try:
+                c = torch.zeros(Ms[-1], N, device="cuda")
+                before = fg.kernel_launches()
+                fg.chain_registered("f32", c, b, N, W)
+                fg.sync()
+                launches = fg.kernel_launches() - before
+            finally:
+                fg.set_chain_mode("fused")
+            assert (launches == 1) == (mode == "fused")
+            out.append(c.cpu().numpy())
+        for w in W:
+            w.release()
+        np.testing.assert_array_equal(out[0], out[1])  # NaN equal to NaN
+        return out[0]
+
+    got = run(As)
+    assert np.isfinite(np.delete(got, [40, 131, 250], axis=1)).all()
+    assert not np.isfinite(got[:, [40, 131]]).any()
+    As[-1][3, 2] = np.inf
+    got = run(As)
+    assert not np.isfinite(got[3]).any() and np.isfinite(np.delete(got, [40, 131, 250], axis=1)[4:]).all()

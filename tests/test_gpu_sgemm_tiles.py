@@ -71,6 +71,31 @@ def test_more_columns_than_a_31_bit_byte_count(N):
         assert torch.equal(c[i], a[i, 0] * b[0] + a[i, 1] * b[1])
 
 
+def test_captured_call_with_k_blocks():
+    """K > 2048 on a stream that is being captured: no workspace, the blocks in turn, and
+    the graph computes from what its operands hold when it runs."""
+    import torch
+    import flashgemm_b200 as fg
+    M, N, K = 35, 457, 4100
+    A, B = oracle.sgemm_inputs(M, N, K, seed=1)
+    a, b = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+    c = torch.zeros(M, N, device="cuda")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    fg.sgemm_dev(c, a, b, M, N, K, stream=s)  # the work is on this stream from here on
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        fg.sgemm_dev(c, a, b, M, N, K, stream=s)
+    for scale in (1.0, -2.0):
+        a.copy_(torch.from_numpy(A) * scale)
+        c.fill_(7.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        want = oracle.sgemm_f32(A * np.float32(scale), B, kblock=2048)
+        np.testing.assert_array_equal(c.cpu().numpy(), want)
+
+
 NO_ROOM = """
 import torch
 import flashgemm_b200 as fg
