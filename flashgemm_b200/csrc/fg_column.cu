@@ -606,12 +606,17 @@ bool column_layout(int n, const long *M, const long *K, ColArgs &A)
 
 }  // namespace
 
-// Clocks of both ways (a model, per the rates measured on B200): here every SM runs
-// whole blocks, a block's stages one after the other (three MMAs per 8 k, about 3000
-// clocks of hand-over per stage), or its share of the memory that B and C cross; the
-// launch-per-stage path splits B through memory (12 bytes a value) and then spreads
-// 128 x 128 tiles of each stage over all SMs, a k-block in about 1400 clocks, a stage's
-// launch and drain about 6000. Deep or tall stages on few columns stay there.
+// Microseconds of both ways, fitted to measurements on B200 of 436 random chains of 2 to 5
+// stages (N = 16 to 65536, K_1 = 16 to 8400, registered weights). Here every SM runs whole
+// blocks, a block's stages one after the other: a k-block of the first stage takes 0.62 (16-deep
+// granules: 0.92), which a few blocks cannot share. The launch-per-stage path splits B
+// through memory (12 bytes a value) and then spreads 128 x 128 tiles of each stage over all
+// SMs, a k-block in 0.52, a stage's launch and drain in 6.6. So deep first stages and tall
+// last ones on few columns stay there. Measured, column / stages: N = 64, K_1 = 3524, rows
+// 32, 792 138 / 72; N = 96, 5276, 20, 560 183 / 102; N = 144, 5276, 48, 36, 268 114 / 117;
+// N = 6624, 3532, 12, 64 77 / 130. The lower one is the faster at all but 5 of the 436, and
+// within 11 % there. First stages of 129 to 144 rows stay here up to 1.5 times the other
+// estimate, for the single launch: N = 640, 2050, 144, 144 82 / 58, N = 900, 864, 130 33 / 25.
 bool column_preferred(long N, int n, const long *M, const long *K, int num_sms)
 {
     if (n < 1 || n > kPanelMaxStages || N < 1 || N > (1l << 30)) return false;
@@ -619,18 +624,20 @@ bool column_preferred(long N, int n, const long *M, const long *K, int num_sms)
         if (M[i] < 1 || K[i] < 1 || M[i] > (1l << 30) || K[i] > (1l << 30)) return false;
     static thread_local ColArgs A;
     if (!column_layout(n, M, K, A)) return false;
-    const double blocks = (double)((N + kCBN - 1) / kCBN);
-    double block = 0.0, staged = 12.0 * K[0] * N / 3300.0;
+    const double blocks = (double)((N + kCBN - 1) / kCBN), mb = 1e-6;
+    const bool whole = A.gran_k == 32, shared = A.small && blocks > num_sms;
+    double block = 0.0, staged = 2.2 + 0.218 * mb * 12.0 * K[0] * N;
     for (int i = 0; i < n; ++i) {
         const ColStage &cs = A.st[i];
-        block += cs.tiles * ((cs.K + 7) / 8 * 3.0 * std::max(48.0, cs.rows / 2.0) + 3000.0);
-        const double tiles = (double)((M[i] + 127) / 128) * blocks;
-        staged += 6000.0 + std::ceil(tiles / num_sms) * ((K[i] + 31) / 32) * 1400.0;
+        const double kb = (cs.K + kCBK - 1) / kCBK;
+        const double per_kb = i > 0 ? 0.71 : !whole ? 0.92 + 0.0004 * cs.rows : shared ? 0.66 : 0.62;
+        block += 0.67 + (cs.tiles - 1) * 0.21 + cs.tiles * (kb * per_kb + 0.0085 * cs.rows);
+        const double waves = std::ceil((double)((M[i] + 127) / 128) * blocks / num_sms);
+        staged += 6.6 + waves * kb * 0.52 + (waves - 1.0) * 2.0 + 0.0104 * mb * 12.0 * M[i] * N;
     }
-    const double per_sm = A.small ? 2.0 : 1.0;
-    const double here = std::max(std::ceil(blocks / (num_sms * per_sm)) * block,
-                                 4.0 * (K[0] + M[n - 1]) * N / 3300.0);
-    return here < staged;
+    const double rounds = std::ceil(blocks / (num_sms * (A.small ? 2.0 : 1.0)));
+    const double here = 3.4 + rounds * block + 0.028 * mb * 4.0 * (K[0] + M[n - 1]) * N;
+    return here < staged * (A.st[0].rows > 128 ? 1.5 : 1.0);
 }
 
 cudaError_t launch_column(const PanelChainArgs &a, int num_sms, int *status, cudaStream_t s)
