@@ -541,14 +541,15 @@ bool narrow_eligible(const StageArgs *st, int n)
     return true;
 }
 
-// Microseconds of both kernels, fitted to measurements on B200 of 19 chains (64,64,64 to
-// 4800,192,56,336 and 64,128,4096) at N = 64 to 65536, registered weights, both types.
-// Narrow: a block's stages one after the other (per stage, per k-block, per row), the
-// blocks of one SM in turn, or two at a time. Fused: a stage's tiles over all CTA pairs.
-// The lower one of the two is within 6 % of the faster everywhere there. Measured, us,
-// narrow / fused: BF16 256,256,256 at N = 9216 12 / 18, at 65536 39 / 41, 64,128,4096 at 64
-// 55 / 12, 4096,128,512 at 20000 68 / 64; INT8 4800,192,56,336 at 4096 22 / 41, 256,256,2048
-// at 1024 38 / 33, 64,128,1024 at 65536 65 / 170.
+// Microseconds of both kernels, fitted to measurements on B200 of 3100 random chains of 2 to
+// 6 stages per type (N = 16 to 65536, K_1 = 16 to 8400, last stage of up to 4096 rows, registered
+// weights). Narrow: a block's stages one after the other (per stage, per k-block, per row, per
+// tile of the last), the blocks of one SM in turn, or two at a time. Fused: a stage's tiles over
+// all CTA pairs; it reads each INT8 tail row's quad per column. (More than 144 rows leave the
+// first stage of a BF16 chain fewer ring slots.) The lower one of the two is the faster, or
+// within 5 % of it, at 99.5 % of them, and within 17 % at the rest. Measured, us, narrow / fused: BF16 256,256,256 at N = 9216 12 / 18, at 65536 39 / 41;
+// 4532,12,2244 at 96 45 / 33; 4472,8,80,16,1288 at 2308 68 / 74; INT8 4800,192,56,336 at 4096
+// 22 / 41; 136,8,80,36,28,28,3156 at 688 42 / 73; 364,232,20,2584 at 16 34 / 23.
 bool narrow_preferred(const StageArgs *st, int n, int num_sms)
 {
     static thread_local NarrowArgs A;
@@ -556,24 +557,25 @@ bool narrow_preferred(const StageArgs *st, int n, int num_sms)
     if (!(i8 ? narrow_layout<OP_I8>(st, n, num_sms, A) : narrow_layout<OP_BF16>(st, n, num_sms, A))) return false;
     const double kb_elems = i8 ? 128.0 : 64.0;
     const long N = st[0].N, pairs = num_sms / 2;
-    double block = i8 ? 0.47 : 0.0, fused = 8.0;
-    bool tails = false;
+    double block = 0.0, fused = i8 ? 5.0 : 4.8;
     for (int i = 0; i < n; ++i) {
-        const double kb = std::ceil(st[i].K / kb_elems), M = st[i].M;
-        if (i + 1 < n)
-            block += i8 ? 0.33 + 0.0134 * M + kb * ((i ? 0.0 : 0.307) + 0.0002 * M)
-                        : 0.07 + 0.0038 * M + kb * ((i ? 0.0 : 0.07) + 0.0013 * M);
+        const double kb = std::ceil(st[i].K / kb_elems), rows = A.st[i].rows;
+        if (i + 1 == n)
+            block += A.st[i].tiles * (i8 ? 1.33 + 0.063 * kb : 1.23 + 0.14 * kb);
+        else if (i8)
+            block += 0.46 + 0.0068 * rows + kb * (i ? 0.354 : 0.317 + 0.00023 * rows);
         else
-            block += i8 ? 0.0115 * M : std::ceil(M / 128.0) * (0.83 + 0.178 * kb);
+            block += 0.64 + 0.0074 * rows + kb * (i ? 0.23 : 0.28 + 0.0014 * std::max(0.0, rows - 144.0));
         const double rounds =
             std::ceil((double)((st[i].M + 255) / 256) * ((N + 255) / 256) / pairs);
-        fused += 3.4 + kb * rounds * (i8 ? 0.25 : 0.3) + (rounds - 1.0) * (i8 ? 4.0 : 3.0);
-        tails = tails || st[i].tail_hi > st[i].tail_lo;
+        fused += i8 ? 4.1 + kb * rounds * 0.33 + (rounds - 1.0) * 4.0
+                    : 4.7 + kb * rounds * 0.29 + (rounds - 1.0) * 5.7;
+        if (st[i].tail_hi > st[i].tail_lo) fused += 10.8 * std::min(1.0, N / 256.0);
     }
-    if (tails) fused += 14.0;  // the fused kernel reads each tail row's quad per tile
     const double rounds = std::ceil((double)((N + kNBN - 1) / kNBN) / num_sms);
     const double again = A.per_sm > 1 ? (i8 ? 0.87 : 1.07) : (i8 ? 1.19 : 1.57);
-    return (i8 ? 2.9 : 8.1) + block * (1.0 + (rounds - 1.0) * again) < fused;
+    const double narrow = (i8 ? 3.2 : 2.8) + block * (1.0 + (rounds - 1.0) * again);
+    return narrow < fused;
 }
 
 namespace {
