@@ -15,30 +15,51 @@ __device__ __forceinline__ float tf32_rne(float f)
     return __uint_as_float(u & 0xffffe000u);
 }
 
+// Whether a matrix is split by 16-byte accesses; one of dense rows is one long row.
+__host__ __device__ __forceinline__ bool split_flat(const SplitJob &j) { return j.ld_in == j.cols && j.ld_out == j.cols; }
+__host__ __device__ __forceinline__ bool split_vec(const SplitJob &j)
+{
+    return (split_flat(j) ? (j.rows * j.cols) % 4 == 0 : ((j.cols | j.ld_in | j.ld_out) & 3) == 0) &&
+           (((uintptr_t)j.in | (uintptr_t)j.hi | (uintptr_t)j.lo) & 15) == 0;
+}
+
 // x = hi + lo + r with hi = rne_tf32(x), lo = rne_tf32(x - hi), |r| <= 2^-22 |x|.
-// Block `part` of `parts` of one matrix. Bound by memory (4 bytes in, 8 out): 16-byte
-// accesses, four of them in flight per thread; a matrix of dense rows is one long row,
-// so that nothing is divided. Measured (B200, the weights and B of 24 grouped FP32
-// chains, two launches): 73 -> 44 us against one value and one 64-bit division per thread
-// and step.
+// Block `part` of `parts` of one matrix. Bound by memory (4 bytes in, 8 out): four accesses
+// in flight per thread, of 16 bytes where rows and pointers allow it. Measured (B200): the
+// weights and B of 24 grouped FP32 chains, two launches, 73 -> 44 us against one value and one
+// 64-bit division per thread and step; a GEMM of 17789 x 252 x 1429 (4-byte accesses) 203 ->
+// 168 against one of them in flight.
 __device__ __forceinline__ void split_rows(const SplitJob &j, long part, long parts)
 {
-    const bool flat = j.ld_in == j.cols && j.ld_out == j.cols;
+    const bool flat = split_flat(j);
     const long cols = flat ? j.rows * j.cols : j.cols;
-    const bool vec = ((cols | (flat ? 0 : j.ld_in | j.ld_out)) & 3) == 0 &&
-                     (((uintptr_t)j.in | (uintptr_t)j.hi | (uintptr_t)j.lo) & 15) == 0;
-    if (!vec) {
-        const long total = j.rows * j.cols;
-        for (long i = part * blockDim.x + threadIdx.x; i < total; i += parts * blockDim.x) {
-            const long r = i / j.cols, c = i - r * j.cols;
-            const float x = j.in[r * j.ld_in + c];
-            const float h = tf32_rne(x);
-            j.hi[r * j.ld_out + c] = h;
-            j.lo[r * j.ld_out + c] = tf32_rne(x - h);
+    constexpr int U = 4;  // accesses in flight
+    if (!split_vec(j)) {
+        const long total = j.rows * j.cols, step = parts * blockDim.x * U;
+        for (long i0 = part * blockDim.x * U + threadIdx.x; i0 < total; i0 += step) {
+            float x[U];
+            long to[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const long i = i0 + u * (long)blockDim.x;
+                to[u] = -1;
+                if (i < total) {
+                    const long r = total >> 32 ? i / j.cols : (uint32_t)i / (uint32_t)j.cols;
+                    const long c = i - r * j.cols;
+                    to[u] = r * j.ld_out + c;
+                    x[u] = j.in[r * j.ld_in + c];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (to[u] < 0) continue;
+                const float h = tf32_rne(x[u]);
+                j.hi[to[u]] = h;
+                j.lo[to[u]] = tf32_rne(x[u] - h);
+            }
         }
         return;
     }
-    constexpr int U = 4;  // 16-byte accesses in flight
     const long row_quads = cols / 4, total = flat ? row_quads : row_quads * j.rows;
     const long step = parts * blockDim.x * U;
     for (long i0 = part * blockDim.x * U + threadIdx.x; i0 < total; i0 += step) {
@@ -88,31 +109,36 @@ __global__ void __launch_bounds__(256) split_tf32_jobs_kernel(const SplitJob *__
     split_rows(j, blockIdx.x, gridDim.x);
 }
 
-// Blocks for the largest matrix of a launch (4096 values per block and step, at most 8
-// blocks per SM).
-static unsigned split_blocks(long max_elems)
+// Blocks that split one matrix in a single step of each.
+long split_blocks(const SplitJob &j)
 {
-    const long blocks = (max_elems + 4095) / 4096;
-    return (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8);
+    const long per_block = split_vec(j) ? 4096 : 1024;
+    return (j.rows * j.cols + per_block - 1) / per_block;
+}
+
+// Blocks per matrix of a launch: what the largest takes, at most 8 per SM.
+static unsigned split_grid(long most)
+{
+    return (unsigned)(most < 148 * 8 ? most : 148 * 8);
 }
 
 cudaError_t launch_split_tf32(const SplitBatch &b, cudaStream_t s)
 {
     long most = 0;
     for (int i = 0; i < b.n; ++i) {
-        const long e = b.job[i].rows * b.job[i].cols;
-        most = e > most ? e : most;
+        const long n = split_blocks(b.job[i]);
+        most = n > most ? n : most;
     }
     if (most < 1) return cudaSuccess;
-    return launch_overlapped(split_tf32_kernel, dim3(split_blocks(most), (unsigned)b.n), 256, 0, s, b);
+    return launch_overlapped(split_tf32_kernel, dim3(split_grid(most), (unsigned)b.n), 256, 0, s, b);
 }
 
-cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long max_elems,
+cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long most_blocks,
                                    cudaStream_t s)
 {
-    if (njobs < 1 || max_elems < 1) return cudaSuccess;
+    if (njobs < 1 || most_blocks < 1) return cudaSuccess;
     if (njobs > 65535) return cudaErrorInvalidValue;
-    split_tf32_jobs_kernel<<<dim3(split_blocks(max_elems), (unsigned)njobs), 256, 0, s>>>(jobs_dev);
+    split_tf32_jobs_kernel<<<dim3(split_grid(most_blocks), (unsigned)njobs), 256, 0, s>>>(jobs_dev);
     return cudaGetLastError();
 }
 

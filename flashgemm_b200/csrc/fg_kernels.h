@@ -371,7 +371,9 @@ struct SplitBatch {
     int n = 0;
 };
 cudaError_t launch_split_tf32(const SplitBatch &b, cudaStream_t s);
-cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long max_elems,
+// most_blocks: the largest split_blocks of the jobs
+long split_blocks(const SplitJob &j);
+cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long most_blocks,
                                    cudaStream_t s);
 
 // Plain FP32 SGEMMs of many independent jobs in one launch (jobs in device

@@ -127,3 +127,24 @@ def test_no_room_for_k_block_sums():
     with the same bits. In a process of its own, which has no workspace from earlier calls."""
     out = subprocess.run([sys.executable, "-c", NO_ROOM], capture_output=True, text=True, timeout=300)
     assert "SAME BITS" in out.stdout, out.stderr[-2000:]
+
+
+@pytest.mark.parametrize("shape", [(300, 64, 333), (17, 20, 66), (2100, 132, 1429), (1, 4, 3)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_tf32_split_of_odd_rows(shape):
+    """3xTF32 with rows of A that 16-byte accesses cannot split: the bits of the same matrix
+    with zero columns up to a multiple of four, which they can."""
+    import torch
+    import flashgemm_b200 as fg
+    M, N, K = shape
+    K4 = (K + 3) // 4 * 4
+    A, B = oracle.sgemm_inputs(M, N, K, seed=M + K)
+    out = []
+    for k in (K, K4):
+        a, b = torch.zeros(M, k, device="cuda"), torch.zeros(k, N, device="cuda")
+        a[:, :K], b[:K] = torch.from_numpy(A), torch.from_numpy(B)
+        c = torch.full((M, N), 7.0, device="cuda")
+        fg.sgemm_dev(c, a, b, M, N, k, algo="3xtf32")
+        fg.sync()
+        out.append(c.cpu().numpy())
+    np.testing.assert_array_equal(out[0], out[1])
