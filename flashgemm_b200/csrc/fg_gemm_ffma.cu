@@ -204,7 +204,11 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
                         const float4 o = *c4;
                         r[0] = o.x + r[0]; r[1] = o.y + r[1]; r[2] = o.z + r[2]; r[3] = o.w + r[3];
                     }
-                    *c4 = make_float4(r[0], r[1], r[2], r[3]);
+                    const float4 v = make_float4(r[0], r[1], r[2], r[3]);
+                    if constexpr (TN == 8)  // past L1 (18720 x 30480 x 48 1401 -> 1335)
+                        __stcg(c4, v);
+                    else
+                        *c4 = v;
                 } else {
 #pragma unroll
                     for (int u = 0; u < 4; ++u)
@@ -273,9 +277,11 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
             }
         } else {
             // the k past K hold zeros for both operands; they are skipped, so that no
-            // extra rounding step (or 0 x infinity) touches the sums
-#pragma unroll 1
-            for (int k = 0; k < K - s * BK; ++k) {
+            // extra rounding step (or 0 x infinity) touches the sums. Whole quads of k first
+            // (18720 x 30480 x 48, 64 x 64 1429 -> 1401); the 64 x 128 tile has no registers for
+            // it, and in the 16 x 64 one it costs the whole slices 10 %.
+            const int rest = K - s * BK, quads = TM * TN < 64 && TM > 2 ? rest / 4 : 0;
+            auto step = [&](int k, const float (&x)[TM]) {
                 unsigned long long bp[TN / 2];
 #pragma unroll
                 for (int j = 0; j < TN / 4; ++j) {
@@ -285,12 +291,34 @@ __device__ __forceinline__ void ffma_tile(const FfmaArgs &p, int m0, int n0, flo
                 }
 #pragma unroll
                 for (int i = 0; i < TM; ++i) {
-                    const int r = ty + i * TY;
-                    const float x = As[r * BK + a_chunk(r, k / 4) * 4 + (k & 3)];
-                    const unsigned long long ap = pack2(x, x);
+                    const unsigned long long ap = pack2(x[i], x[i]);
 #pragma unroll
                     for (int j = 0; j < TN / 2; ++j) ffma2(acc[i][j], ap, bp[j]);
                 }
+            };
+#pragma unroll 1
+            for (int q = 0; q < quads; ++q) {
+                float4 v[TM];
+#pragma unroll
+                for (int i = 0; i < TM; ++i) v[i] = a_quad(i, q);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float x[TM];
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+                        x[i] = u == 0 ? v[i].x : u == 1 ? v[i].y : u == 2 ? v[i].z : v[i].w;
+                    step(q * 4 + u, x);
+                }
+            }
+#pragma unroll 1
+            for (int k = quads * 4; k < rest; ++k) {
+                float x[TM];
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const int r = ty + i * TY;
+                    x[i] = As[r * BK + a_chunk(r, k / 4) * 4 + (k & 3)];
+                }
+                step(k, x);
             }
         }
         buf = buf + 1 == ST ? 0 : buf + 1;
@@ -402,17 +430,19 @@ using Tiny = Shape<16, 64, 32, 2, 4, 3, 5>;
 // The tile shapes: CTAs resident per SM, and FMA per clock that an SM reaches with
 // one CTA and with all of them (B200; from 256 x 256 x 2048, which gives every shape
 // at most one CTA per SM, and from 1632 x 36548 x 1024).
+// rest: what a k past the last whole slice of 32 costs, in k of a whole one (18720 x 30480 x
+// 40, 48, 64: Wide 1333, 1637, 1589, Square 1160, 1335, 1597).
 struct ShapeInfo {
     int bm, bn, occ;
-    double one, full;
+    double one, full, rest;
 };
 constexpr ShapeInfo kShapes[] = {
-    {64, 128, Wide::OCC, 78.5, 87.9},   // Wide: the best rate; 128 x 128 (8 x 16 per thread) gains nothing on
+    {64, 128, Wide::OCC, 78.5, 87.9, 2.0},   // Wide: the best rate; 128 x 128 (8 x 16 per thread) gains nothing on
                                 // it and leaves the SMs idle at both ends of a short K
-    {64, 64, Square::OCC, 61.0, 83.9},    // Square: two or three per SM where Wide leaves SMs idle
-    {40, 64, Low::OCC, 48.0, 79.8},    // Low: few rows, and dimensions that 64 pads
-    {32, 64, Small::OCC, 43.5, 72.7},    // Small: more CTAs where outputs are few
-    {16, 64, Tiny::OCC, 28.8, 40.0},    // Tiny: at most one CTA per SM
+    {64, 64, Square::OCC, 61.0, 83.9, 1.0},    // Square: two or three per SM where Wide leaves SMs idle
+    {40, 64, Low::OCC, 48.0, 79.8, 1.0},    // Low: few rows, and dimensions that 64 pads
+    {32, 64, Small::OCC, 43.5, 72.7, 1.0},    // Small: more CTAs where outputs are few
+    {16, 64, Tiny::OCC, 28.8, 40.0, 1.0},    // Tiny: at most one CTA per SM
 };
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
@@ -435,13 +465,14 @@ double shape_cost(const ShapeInfo &s, long tiles, int num_sms)
 }
 
 // The cheapest shape for `blocks` K blocks side by side (1: none apart), and its cost.
-int pick_shape(long M, long N, double blocks, int num_sms, double &cost)
+int pick_shape(long M, long N, long K, double blocks, int num_sms, double &cost)
 {
     int best = 0;
+    const double rest = K > 16 ? (double)(K % 32) / K : 0.0;  // fewer: a tile's fixed cost counts more
     for (int i = 0; i < kNumShapes; ++i) {
         const ShapeInfo &s = kShapes[i];
         const double tiles = (double)((M + s.bm - 1) / s.bm) * ((N + s.bn - 1) / s.bn);
-        const double c = shape_cost(s, (long)(tiles * blocks + 0.999), num_sms);
+        const double c = shape_cost(s, (long)(tiles * blocks + 0.999), num_sms) * (1.0 + (s.rest - 1.0) * rest);
         if (i == 0 || c < cost) {
             best = i;
             cost = c;
@@ -547,8 +578,8 @@ size_t ffma_sgemm_workspace(long M, long N, long K, int kblock, int num_sms)
     const double part_bytes = (double)(blocks - 1) * M * ld * 4;
     if (part_bytes > (double)(1l << 30)) return 0;  // such results fill the SMs anyhow
     double whole = 0.0, apart = 0.0;
-    pick_shape(M, N, 1.0, num_sms, whole);
-    pick_shape(M, N, (double)K / kblock, num_sms, apart);
+    pick_shape(M, N, K, 1.0, num_sms, whole);
+    pick_shape(M, N, K, (double)K / kblock, num_sms, apart);
     // clocks: 6000 for the launch, the parts written and read once at 3000 bytes a clock
     return apart * kblock + 6000.0 + 2.0 * part_bytes / 3000.0 < whole * K ? (size_t)part_bytes : 0;
 }
@@ -559,7 +590,7 @@ cudaError_t launch_ffma_sgemm(const FfmaArgs &a, int num_sms, cudaStream_t s)
     if (a.kblock > 0 && a.kblock % 32) return cudaErrorInvalidValue;  // K blocks end on slices
     double cost = 0.0;
     const int shape = forced_shape() >= 0 ? forced_shape()
-                                          : pick_shape(a.M, a.N, a.part ? (double)a.K / a.kblock : 1.0,
+                                          : pick_shape(a.M, a.N, a.K, a.part ? (double)a.K / a.kblock : 1.0,
                                                        num_sms, cost);
     cudaError_t e;
     switch (shape) {
