@@ -28,13 +28,15 @@ __host__ __device__ __forceinline__ bool split_vec(const SplitJob &j)
 // in flight per thread, of 16 bytes where rows and pointers allow it. Measured (B200): the
 // weights and B of 24 grouped FP32 chains, two launches, 73 -> 44 us against one value and one
 // 64-bit division per thread and step; a GEMM of 17789 x 252 x 1429 (4-byte accesses) 203 ->
-// 168 against one of them in flight.
+// 168 against one of them in flight. MIXED: some matrix of the launch needs 4-byte accesses
+// (together the two loops take more registers, and 3 % of the time, than the one).
+template <bool MIXED>
 __device__ __forceinline__ void split_rows(const SplitJob &j, long part, long parts)
 {
     const bool flat = split_flat(j);
     const long cols = flat ? j.rows * j.cols : j.cols;
     constexpr int U = 4;  // accesses in flight
-    if (!split_vec(j)) {
+    if (MIXED && !split_vec(j)) {
         const long total = j.rows * j.cols, step = parts * blockDim.x * U;
         for (long i0 = part * blockDim.x * U + threadIdx.x; i0 < total; i0 += step) {
             float x[U];
@@ -97,48 +99,50 @@ __device__ __forceinline__ void split_rows(const SplitJob &j, long part, long pa
 
 // A few matrices in one launch, blockIdx.y = job, the jobs in the parameters or in
 // device memory.
+template <bool MIXED>
 __global__ void __launch_bounds__(256) split_tf32_kernel(const __grid_constant__ SplitBatch b)
 {
     overlap_next();
     overlap_wait();
-    split_rows(b.job[blockIdx.y], blockIdx.x, gridDim.x);
+    split_rows<MIXED>(b.job[blockIdx.y], blockIdx.x, gridDim.x);
 }
+template <bool MIXED>
 __global__ void __launch_bounds__(256) split_tf32_jobs_kernel(const SplitJob *__restrict__ jobs)
 {
     const SplitJob j = jobs[blockIdx.y];
-    split_rows(j, blockIdx.x, gridDim.x);
+    split_rows<MIXED>(j, blockIdx.x, gridDim.x);
 }
 
-// Blocks that split one matrix in a single step of each.
-long split_blocks(const SplitJob &j)
+void SplitSize::add(const SplitJob &j)
 {
-    const long per_block = split_vec(j) ? 4096 : 1024;
-    return (j.rows * j.cols + per_block - 1) / per_block;
+    const bool vec = split_vec(j);
+    const long per_block = vec ? 4096 : 1024;
+    const long n = (j.rows * j.cols + per_block - 1) / per_block;
+    blocks = n > blocks ? n : blocks;
+    mixed = mixed || !vec;
 }
 
 // Blocks per matrix of a launch: what the largest takes, at most 8 per SM.
-static unsigned split_grid(long most)
-{
-    return (unsigned)(most < 148 * 8 ? most : 148 * 8);
-}
+static unsigned split_grid(const SplitSize &z) { return (unsigned)(z.blocks < 148 * 8 ? z.blocks : 148 * 8); }
 
 cudaError_t launch_split_tf32(const SplitBatch &b, cudaStream_t s)
 {
-    long most = 0;
-    for (int i = 0; i < b.n; ++i) {
-        const long n = split_blocks(b.job[i]);
-        most = n > most ? n : most;
-    }
-    if (most < 1) return cudaSuccess;
-    return launch_overlapped(split_tf32_kernel, dim3(split_grid(most), (unsigned)b.n), 256, 0, s, b);
+    SplitSize z;
+    for (int i = 0; i < b.n; ++i) z.add(b.job[i]);
+    if (z.blocks < 1) return cudaSuccess;
+    return launch_overlapped(z.mixed ? split_tf32_kernel<true> : split_tf32_kernel<false>,
+                             dim3(split_grid(z), (unsigned)b.n), 256, 0, s, b);
 }
 
-cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long most_blocks,
-                                   cudaStream_t s)
+cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, const SplitSize &z, cudaStream_t s)
 {
-    if (njobs < 1 || most_blocks < 1) return cudaSuccess;
+    if (njobs < 1 || z.blocks < 1) return cudaSuccess;
     if (njobs > 65535) return cudaErrorInvalidValue;
-    split_tf32_jobs_kernel<<<dim3(split_grid(most_blocks), (unsigned)njobs), 256, 0, s>>>(jobs_dev);
+    const dim3 grid(split_grid(z), (unsigned)njobs);
+    if (z.mixed)
+        split_tf32_jobs_kernel<true><<<grid, 256, 0, s>>>(jobs_dev);
+    else
+        split_tf32_jobs_kernel<false><<<grid, 256, 0, s>>>(jobs_dev);
     return cudaGetLastError();
 }
 

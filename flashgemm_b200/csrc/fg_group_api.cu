@@ -349,7 +349,7 @@ int group_build(DevCtx *c, int dtype, int algo, int kernel, int order, int nchai
             float *xh = (float *)cv.take((size_t)K[0] * ldN * 4);
             float *xl = (float *)cv.take((size_t)K[0] * ldN * 4);
             gx.splits.push_back(SplitJob{(const float *)d.B, N, xh, xl, ldN, K[0], N});
-            gx.split_most = std::max(gx.split_most, split_blocks(gx.splits.back()));
+            gx.split_size.add(gx.splits.back());
             float *ph[2] = {nullptr, nullptr}, *pl[2] = {nullptr, nullptr};
             if (n > 1)
                 for (int q = 0; q < 2; ++q) {
@@ -506,7 +506,7 @@ int group_launch(DevCtx *c, const GroupExec &gx, cudaStream_t s, bool capturing,
     if (gx.done_ints) CUDA_TRY(cudaMemsetAsync(gx.done, 0, gx.done_ints * sizeof(int), s));
     if (!gx.splits.empty()) {
         int st = run_kernel_on(c, s, capturing, FG_PK_AUX, 0.0, "tf32 split (group)", [&] {
-            return launch_split_tf32_jobs(gx.splits_dev, (int)gx.splits.size(), gx.split_most, s);
+            return launch_split_tf32_jobs(gx.splits_dev, (int)gx.splits.size(), gx.split_size, s);
         });
         if (st) return st;
     }

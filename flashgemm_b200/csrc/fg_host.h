@@ -276,7 +276,7 @@ struct GroupExec {
     std::vector<void *> tables;        // device copies of gls[i].tables
     std::vector<SplitJob> splits;      // 3xTF32: activation splits before the group
     SplitJob *splits_dev = nullptr;
-    long split_most = 0;               // blocks for the largest of them
+    SplitSize split_size;
     struct Level {
         std::vector<FfmaJob> jobs;
         FfmaJob *dev = nullptr;

@@ -371,9 +371,13 @@ struct SplitBatch {
     int n = 0;
 };
 cudaError_t launch_split_tf32(const SplitBatch &b, cudaStream_t s);
-// most_blocks: the largest split_blocks of the jobs
-long split_blocks(const SplitJob &j);
-cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, long most_blocks,
+// What a launch of several needs: every job is added.
+struct SplitSize {
+    long blocks = 0;     // that split the largest in one step of each
+    bool mixed = false;  // some job's rows or pointers are not 16-byte aligned
+    void add(const SplitJob &j);
+};
+cudaError_t launch_split_tf32_jobs(const SplitJob *jobs_dev, int njobs, const SplitSize &size,
                                    cudaStream_t s);
 
 // Plain FP32 SGEMMs of many independent jobs in one launch (jobs in device
