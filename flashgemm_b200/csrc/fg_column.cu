@@ -615,8 +615,9 @@ bool column_layout(int n, const long *M, const long *K, ColArgs &A)
 // last ones on few columns stay there. Measured, column / stages: N = 64, K_1 = 3524, rows
 // 32, 792 138 / 72; N = 96, 5276, 20, 560 183 / 102; N = 144, 5276, 48, 36, 268 114 / 117;
 // N = 6624, 3532, 12, 64 77 / 130. The lower one is the faster at all but 5 of the 436, and
-// within 11 % there. First stages of 129 to 144 rows stay here up to 1.5 times the other
-// estimate, for the single launch: N = 640, 2050, 144, 144 82 / 58, N = 900, 864, 130 33 / 25.
+// within 11 % there. First stages of 129 to 144 rows and K_1 <= 2080 stay here up to 1.5 times
+// the other estimate, in one launch as tests/test_gpu_column.py has them: N = 640, 2050, 144,
+// 144 82 / 58, N = 900, 864, 130 33 / 25.
 bool column_preferred(long N, int n, const long *M, const long *K, int num_sms)
 {
     if (n < 1 || n > kPanelMaxStages || N < 1 || N > (1l << 30)) return false;
@@ -637,7 +638,7 @@ bool column_preferred(long N, int n, const long *M, const long *K, int num_sms)
     }
     const double rounds = std::ceil(blocks / (num_sms * (A.small ? 2.0 : 1.0)));
     const double here = 3.4 + rounds * block + 0.028 * mb * 4.0 * (K[0] + M[n - 1]) * N;
-    return here < staged * (A.st[0].rows > 128 ? 1.5 : 1.0);
+    return here < staged * (A.st[0].rows > 128 && K[0] <= 2080 ? 1.5 : 1.0);
 }
 
 cudaError_t launch_column(const PanelChainArgs &a, int num_sms, int *status, cudaStream_t s)
