@@ -26,10 +26,9 @@
 // products where it fits, one commit per k-block, and waits tested ahead; and, on many
 // columns, reading B once. The launch-per-stage path that it replaces wrote B's split to
 // memory and read it back (3x its bytes) and paid a launch and a memory round trip per
-// stage. Measured (B200, us a call, that
-// path -> this): 12544 x 864, 96, 24, 144 102 -> 33; 65536 x 288, 32, 24, 144 159 -> 53;
-// 50176 x 288, 32, 16, 96 121 -> 41; 16384 x 1296, 144, 32, 192 181 -> 64; 3136 x the same
-// 81 -> 60.
+// stage. Measured (B200, us a call, weights split per call, that path -> this): 12544 x 864,
+// 96, 24, 144 102 -> 33; 65536 x 288, 32, 24, 144 163 -> 49; 50176 x 288, 32, 16, 96 125 ->
+// 38; 16384 x 1296, 144, 32, 192 185 -> 63; 3136 x the same 80 -> 59.
 //
 // The arithmetic is that path's: per 8 k the correction terms lo * hi, then hi * lo,
 // into their own accumulator and hi * hi into the chunk's (hi * [hi | lo] as one MMA over the

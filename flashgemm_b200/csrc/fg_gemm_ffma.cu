@@ -28,9 +28,9 @@
 // memory instead of in registers (1.2-1.4x slower: twice the shared-memory
 // reads), pairs along the diagonal (no faster), scalar FMAs (0.9x), registers
 // between global and shared memory instead of cp.async (the kernel before this
-// one). Before and now, us a call (B200): 1024^3 79 -> 58 (27 -> 37 TFLOP/s),
-// 1632 x 36548 x 1024 2693 -> 2410 (51 TFLOP/s), 35 x 8457 x 2560 141 -> 86,
-// 512 x 289 x 1024 65 -> 29, 4096^3 3577 -> 2588.
+// one). Before and now, us a call (B200): 1024^3 80 -> 58 (27 -> 37 TFLOP/s),
+// 1632 x 36548 x 1024 2694 -> 2402 (51 TFLOP/s), 35 x 8457 x 2560 142 -> 77,
+// 512 x 289 x 1024 66 -> 29, 4096^3 3580 -> 2566.
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -442,7 +442,7 @@ constexpr ShapeInfo kShapes[] = {
     {64, 64, Square::OCC, 61.0, 83.9, 1.0},    // Square: two or three per SM where Wide leaves SMs idle
     {40, 64, Low::OCC, 48.0, 79.8, 1.0},    // Low: few rows, and dimensions that 64 pads
     {32, 64, Small::OCC, 43.5, 72.7, 1.0},    // Small: more CTAs where outputs are few
-    {16, 64, Tiny::OCC, 28.8, 40.0, 1.0},    // Tiny: at most one CTA per SM
+    {16, 64, Tiny::OCC, 28.8, 40.0, 1.0},    // Tiny: few outputs, so many CTAs
 };
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
@@ -567,8 +567,8 @@ cudaError_t launch_ffma_group(const FfmaJob *jobs_dev, int njobs, int total_tile
 // a second kernel adds them in order: the same bits. That costs the launch (about
 // 3 us) and the parts' traffic; it is taken where the tiles' cost falls by more.
 // Measured (B200, us a call; first figure: the kernel before this tile, which could not):
-// 128 x 2048 x 4096 276 -> 72, 84 x 1024 x 4096 303 -> 45, 35 x 8457 x 2560 141 -> 86,
-// 1024 x 16 x 500000 38000 -> 1436.
+// 128 x 2048 x 4096 277 -> 70, 84 x 1024 x 4096 304 -> 47, 35 x 8457 x 2560 142 -> 77,
+// 1024 x 16 x 500000 38100 -> 1435.
 size_t ffma_sgemm_workspace(long M, long N, long K, int kblock, int num_sms)
 {
     if (M <= 0 || N <= 0 || kblock <= 0 || K <= kblock) return 0;

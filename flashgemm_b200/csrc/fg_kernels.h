@@ -20,14 +20,16 @@ namespace fg {
 __device__ __forceinline__ void overlap_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void overlap_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// kernel<<<grid, block, smem, s>>>(args...), allowed to begin early. Only for kernels whose
-// CTAs do not wait on one another (two such grids may hold parts of the device at once)
-// and that fill an SM with one CTA, or all SMs: CTAs placed while the kernel before still
-// runs go where there is room, not evenly (the FP32 SGEMM, several small CTAs per SM,
-// ran 1024^3 in 76 instead of 58 us so). Hides the launch and the prologue (barriers,
-// tensor maps, TMEM): measured (B200, us a call) 28.6 -> 25.7 (BF16 chain 16384 x 1296, 144,
-// 32, 192), 41.0 -> 36.7 (INT8 chain 4096 x 4800, 192, 56, 336, a preparation and a
-// chain kernel), 36.9 -> 32.8 (FP32 chain 12544 x 864, 96, 24, 144, the same).
+// kernel<<<grid, block, smem, s>>>(args...), allowed to begin early: only for kernels whose
+// CTAs do not wait on one another. CTAs placed while the kernel before still runs go where
+// there is room, not evenly, which costs a kernel of several long CTAs per SM more than the
+// launch (the FP32 SGEMM ran 1024^3 in 76 instead of 58 us so); it does not matter to short
+// memory-bound ones (splits, preparations, the sum of K blocks), nor to the on-chip chains,
+// whose grid is one CTA per column block or fills every SM with one or two. Hides the
+// launch and the prologue (barriers, tensor maps, TMEM): measured (B200, us a call) 18.5 ->
+// 17.0 (BF16 chain 16384 x 1296, 144, 32, 192), 30.7 -> 25.1 (INT8 chain 4096 x 4800, 192, 56,
+// 336, a preparation and a chain kernel), 36.9 -> 32.9 (FP32 chain 12544 x 864, 96, 24,
+// 144, a split and a chain kernel).
 template <class... P, class... A>
 cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s,
                               A &&...args)

@@ -16,8 +16,8 @@
 // KB of activations (later stages: none, A is in TMEM) and 32 bytes per real row.
 // Measured (B200, us a call, before -> now; before, the rows were the MMA's M and the
 // intermediates lay in shared memory): BF16 16384 x 1296, 144, 32, 192 24.1 -> 16.9, INT8
-// 4096 x 4800, 192, 56, 336 37.0 -> 24.9; 65536 x 288, 32, 24, 144 33 -> 22.5 (BF16), 30 ->
-// 17.8 (INT8); 20000 x 64, 128, 1024 33 -> 31 (BF16), 40 -> 31 (INT8). What is left there:
+// 4096 x 4800, 192, 56, 336 37.0 -> 25.0; 65536 x 288, 32, 24, 144, registered, 36 -> 22
+// (BF16), 33 -> 18 (INT8); 20000 x 64, 128, 1024 37 -> 30 (BF16), 43 -> 29 (INT8). What is left:
 // the first stage's k-blocks come from L2 at 13 TB/s (BF16 table chain), or 32 blocks leave
 // 116 SMs idle (INT8; its k-blocks shared by a cluster of four CTAs, sums exchanged over
 // distributed shared memory, took 26.8 us: the exchange costs what the split saves).

@@ -331,10 +331,6 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
     }
 }
 
-// Two-CTA MMA, issued by one thread of the pair's first CTA: A rows 0-127 and
-// B columns [0, N/2) come from this CTA's shared memory, A rows 128-255 and B
-// columns [N/2, N) from the peer's at the same offsets; D rows 0-127 land in
-// this CTA's TMEM, rows 128-255 in the peer's, at the same TMEM address.
 // TF32 with the A operand in TMEM: 128 lanes (rows of A), 8 columns (k) at a_tmem; the
 // descriptor of B by its two words.
 __device__ __forceinline__ void tc_mma_ts_tf32(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo,
@@ -363,6 +359,10 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint
             "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate));
 }
 
+// Two-CTA MMA, issued by one thread of the pair's first CTA: A rows 0-127 and
+// B columns [0, N/2) come from this CTA's shared memory, A rows 128-255 and B
+// columns [N/2, N) from the peer's at the same offsets; D rows 0-127 land in
+// this CTA's TMEM, rows 128-255 in the peer's, at the same TMEM address.
 template <MmaKind K>
 __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                             uint32_t idesc, uint32_t accumulate)

@@ -75,7 +75,7 @@ int fg_get_chain_mode(void);
 
 /* Fused BF16 / INT8 chains whose intermediates have at most 256 rows can keep
  * them on chip (the narrow chain kernel: one CTA per 128-column block, each
- * intermediate narrowed and permuted straight into shared memory; same
+ * intermediate narrowed and permuted straight into tensor memory; same
  * results as the other paths).
  * FG_NARROW_AUTO (default): where a model fitted to measurements expects it to be
  *   faster (most chains but those with a wide last stage or a deep first stage
@@ -102,7 +102,10 @@ int fg_chain_dev(int dtype, void *C, const void *B, long N, int num_gemm, const 
 
 /* C = A * B on device memory (row-major, dense leading dimensions), with the
  * given FP32 algorithm (FG_F32_FFMA or FG_F32_3XTF32). Asynchronous like
- * fg_chain_dev. */
+ * fg_chain_dev. With FG_F32_FFMA and K > 2048 the blocks of 2048 k run side by
+ * side where that pays, in a workspace that the library keeps (at most 1.4 GB; given
+ * back when its scratch cannot grow otherwise); where it cannot be had, or the stream
+ * is being captured, they run in turn, with the same bits. */
 int fg_sgemm_dev(float *C, const float *A, const float *B, long M, long N, long K, int algo,
                  void *stream);
 
@@ -204,10 +207,11 @@ int fg_group_choice(int dtype, int nchains, const fg_chain_desc *chains, int *ke
  * weights are admitted in arrival order while the device-memory budget and a
  * launch slot allow, packed into grouped launches (one per dtype present) and
  * run on one of `slots` streams, so a batch admitted while others are still on
- * the GPU overlaps with them (each batch's persistent grids are capped at
- * SMs / slots CTAs unless ctas_per_batch says otherwise; a batch launched while
- * none is in flight may take every SM, and one that follows starts as its CTAs
- * leave). The device is never
+ * the GPU overlaps with them. A batch's launches run side by side, each of at
+ * most SMs / slots CTAs unless ctas_per_batch says otherwise (all SMs where no
+ * other batch is in flight; one that follows starts as its CTAs leave). Where a
+ * kernel's CTAs wait on one another (FG_GROUP_PAIR), the batch's launches run in
+ * turn, and none beside them takes more than its share. The device is never
  * left idle while requests wait: a batch is launched at once when no other is
  * in flight, else when it holds max_batch requests or its oldest request has
  * waited max_wait_us. Results are the ones fg_chain_registered gives for the
